@@ -231,6 +231,32 @@ void free_block(BlockH& b) {
 // 1.358, 1.379 ms).
 constexpr int STREAM_STRIP_ROWS = 4;
 
+// Rows of an FP64 update item (32 columns each, knc_f64_update.cu) where the
+// caller has not chosen them. The update's time is the FP64 instructions of
+// the SM that gets the most CTAs (4 items each): an item costs about one row's
+// instructions before its march (the edges and the first face) and then one
+// per row, and a CTA alone on its SM runs a fifth slower (nothing hides its
+// other instructions). The rows that make that least.
+int64_t f64_update_rows(const std::vector<std::pair<int64_t, int64_t>>& shapes, int sms) {
+    int64_t best = 1;
+    double least = -1.0;
+    for (int64_t rows = 1; rows <= 32; ++rows) {
+        int64_t items = 0, most = 0;
+        for (const auto& s : shapes) {
+            const int64_t per = (s.first + rows - 1) / rows;
+            items += per * ((s.second + TILE_Q - 1) / TILE_Q);
+            most = std::max(most, (s.first + per - 1) / per);
+        }
+        const int64_t ctas = (items + 3) / 4, on_sm = (ctas + sms - 1) / sms;
+        const double cost = (double)on_sm * ((double)most + 1.1) * (on_sm == 1 ? 1.2 : 1.0);
+        if (least < 0.0 || cost < least) {
+            least = cost;
+            best = rows;
+        }
+    }
+    return best;
+}
+
 // One block set's device view.
 struct Layout {
     DevBlock* d_table = nullptr;
@@ -243,6 +269,8 @@ struct Layout {
     int nutiles = 0;
     int utr = 0;
     int uform = -1;
+    int list_cols = 0;          // columns of a strip: 32 for the FP64 update's items, else STRIP_OUT
+    bool list_auto = false;     // item rows by f64_update_rows
     int64_t nzones = 0;         // zones of the block set
     TmaMaps* d_tmaps = nullptr; // tensor maps per slot (tiles of `utr` rows), when every block allows them
     int tmaps_cap = 0;
@@ -377,6 +405,7 @@ struct knc_ctx {
     int32_t guess = KNC_GUESS_PLAIN;
     int32_t batched = 0;
     int32_t utr = 8;   // update tile rows (4, 8 or 16)
+    bool utr_set = false;   // chosen by the caller or the autotuner
     int32_t fused = 0;         // one cooperative launch per stage
     int32_t uform = KNC_UPDATE_TILE;   // update form of the separate stage
     int32_t rform = KNC_RECOVERY_INLINE;   // mixed recovery form of the separate stage
@@ -629,8 +658,21 @@ int fused_threads(const knc_ctx* c) {
 
 // Rebuild the device block table and the tile list after the block set changed.
 int rebuild_table(knc_ctx* c) {
-    if (!c->dirty && L(c).utr == c->utr && L(c).uform == c->uform && L(c).chunk_nt == fused_threads(c))
+    // the separate FP64 update takes items of 32 whole columns and at most 32
+    // rows, in both update forms
+    const bool rows64 = c->precision != KNC_PRECISION_MIXED && !c->fused;
+    const bool rows_auto = rows64 && !c->utr_set;
+    const int cols = rows64 ? TILE_Q : STRIP_OUT;
+    if (!c->dirty && L(c).utr == c->utr && L(c).uform == c->uform && L(c).chunk_nt == fused_threads(c) &&
+        L(c).list_cols == cols && L(c).list_auto == rows_auto)
         return KNC_OK;
+    std::vector<std::pair<int64_t, int64_t>> shapes;
+    for (auto& kv : c->blocks) shapes.push_back({kv.second.nr, kv.second.nq});
+    const int64_t auto_rows = rows64 ? f64_update_rows(shapes, c->sms) : 0;
+    const int64_t item_rows = rows_auto ? auto_rows : rows64 ? std::min<int64_t>(c->utr, 32) : c->utr;
+    const int64_t stream_rows = rows64 ? auto_rows : STREAM_STRIP_ROWS;
+    L(c).list_cols = cols;
+    L(c).list_auto = rows_auto;
     const int nb = (int)c->blocks.size();
     std::vector<DevBlock> tab(nb);
     std::vector<int4> tiles, utiles, chunks, strips;
@@ -703,27 +745,30 @@ int rebuild_table(knc_ctx* c) {
         L(c).strip_off.push_back((int)strips.size());
         L(c).sstrip_off.push_back((int)sstrips.size());
         L(c).zone_off.push_back(zoff);
-        for (int64_t j0 = 0; j0 < b.nq; j0 += STRIP_OUT)
-            for (int64_t i0 = 0; i0 < b.nr; i0 += STREAM_STRIP_ROWS)
-                sstrips.push_back(
-                    make_int4(slot, (int)i0, (int)j0, (int)std::min<int64_t>(STREAM_STRIP_ROWS, b.nr - i0)));
+        // (FP64: as even as whole rows allow)
+        const int64_t sper = (b.nr + stream_rows - 1) / stream_rows, sh = rows64 ? (b.nr + sper - 1) / sper : stream_rows;
+        for (int64_t j0 = 0; j0 < b.nq; j0 += cols)
+            for (int64_t i0 = 0; i0 < b.nr; i0 += sh)
+                sstrips.push_back(make_int4(slot, (int)i0, (int)j0, (int)std::min<int64_t>(sh, b.nr - i0)));
         for (int64_t i0 = 0; i0 < b.nr; i0 += TILE_R)
             for (int64_t j0 = 0; j0 < b.nq; j0 += TILE_Q)
                 tiles.push_back(make_int4(slot, (int)i0, (int)j0, (int)zoff));
         if (c->uform == KNC_UPDATE_STRIP) {
             // ceil(nr / utr) strips per column, their heights as even as
             // whole rows allow (64 rows at utr 13: 13, 13, 13, 13, 12)
-            const int64_t per = (b.nr + c->utr - 1) / c->utr;
-            for (int64_t j0 = 0; j0 < b.nq; j0 += STRIP_OUT)
+            const int64_t per = (b.nr + item_rows - 1) / item_rows;
+            for (int64_t j0 = 0; j0 < b.nq; j0 += cols)
                 for (int64_t k = 0, i0 = 0; k < per; ++k) {
                     const int64_t rows = b.nr / per + (k < b.nr % per ? 1 : 0);
                     strips.push_back(make_int4(slot, (int)i0, (int)j0, (int)rows));
                     i0 += rows;
                 }
         } else {
-            for (int64_t i0 = 0; i0 < b.nr; i0 += c->utr)
+            const int64_t per = (b.nr + item_rows - 1) / item_rows;
+            const int64_t th = rows_auto ? (b.nr + per - 1) / per : item_rows;
+            for (int64_t i0 = 0; i0 < b.nr; i0 += th)
                 for (int64_t j0 = 0; j0 < b.nq; j0 += TILE_Q)
-                    utiles.push_back(make_int4(slot, (int)i0, (int)j0, 0));
+                    utiles.push_back(make_int4(slot, (int)i0, (int)j0, (int)std::min<int64_t>(th, b.nr - i0)));
         }
         if (tma_ok) tma_ok = c->utr <= 16 && encode_block_maps(b, c->utr, &maps[k]);
         for (int64_t z0 = 0; z0 < b.nr * b.nq; z0 += nt)
@@ -2313,7 +2358,7 @@ int build_chunks(knc_ctx* c, int S) {
             for (int n : of_chunk[k]) {
                 const Shadow& x = sh[n];
                 const int i0 = x.upper ? 0 : 2 * s + 2;
-                for (int j0 = 0; j0 < tab[x.src].nq; j0 += STRIP_OUT)
+                for (int j0 = 0; j0 < tab[x.src].nq; j0 += l.list_cols)
                     strips.push_back(make_int4(nb + n, i0, j0, rows));
             }
         }
@@ -2685,6 +2730,7 @@ int knc_set_tuning(knc_ctx* c, const knc_tuning* t) {
     if (t->fused && !c->coop)
         return set_msg(c, KNC_ERR_UNSUPPORTED, "the device has no cooperative launch (fused stage)");
     c->utr = t->tile_rows;
+    c->utr_set = true;
     c->fused = t->fused ? 1 : 0;
     c->ctas_per_sm = t->ctas_per_sm;
     // the fused stage stages its tiles itself (no tensor-copy form)
@@ -2772,6 +2818,7 @@ int knc_autotune(knc_ctx* c, int32_t reps, knc_tuning* best_out, double* ms_out)
     for (size_t ci = 0; ci < cands.size(); ++ci) {
         const knc_tuning t = cands[ci];
         c->utr = t.tile_rows;
+        c->utr_set = true;
         c->fused = t.fused;
         c->ctas_per_sm = t.ctas_per_sm;
         c->uform = t.update_form;
@@ -2815,6 +2862,7 @@ int knc_autotune(knc_ctx* c, int32_t reps, knc_tuning* best_out, double* ms_out)
     c->stage_counter = 0;
     c->bar_epoch = 0;
     c->utr = best.tile_rows;
+    c->utr_set = true;
     c->fused = best.fused;
     c->ctas_per_sm = best.ctas_per_sm;
     c->uform = best.update_form;

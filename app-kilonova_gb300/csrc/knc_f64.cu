@@ -6,7 +6,8 @@
 //               time-step reduction of State::time_step (src/state.rs:151-160)
 //   ghost       the two ghost blocks' halo rows from the model at the stage
 //               time (src/scheme.rs:45-52 via BlockState::from_model)
-//   update      flux / source / update / RK average (knc_stage.cuh)
+//   update      flux / source / update / RK average: knc_f64_update.cu (the
+//               fused stage's: knc_stage.cuh)
 //   init        State::from_model (src/state.rs:55-69, 107-115)
 // Without FMA contraction every expression rounds exactly like the CPU
 // oracle's, so this path reproduces the reference arithmetic bit for bit
@@ -17,6 +18,7 @@
 #include "knc_mlp.cuh"
 #include "knc_models.cuh"
 #include "knc_physics.cuh"
+#include "knc_physics64.cuh"
 #include "knc_stage.cuh"
 
 namespace knc {
@@ -34,14 +36,11 @@ struct F64C2p {
         const int nr = B.nr, nq = B.nq;
         const int64_t n = (int64_t)nr * nq;
         const int64_t z = (int64_t)i * nq + j;
-        double u[4] = {1.0, 0.0, 0.0, 1.0};
-        double smass = 0.0, dV = 1.0;
+        double u[5] = {1.0, 0.0, 0.0, 1.0, 0.0};
         if (active) {
-            const double* U = B.buf[a.sel_in];
-            dV = B.dv[z];
-#pragma unroll
-            for (int q = 0; q < 4; ++q) u[q] = U[q * n + z] / dV;
-            smass = U[4 * n + z];
+            const double* Ub = B.buf[a.sel_in] + z;
+            const double U[5] = {Ub[0], Ub[n], Ub[2 * n], Ub[3 * n], Ub[4 * n]};
+            per_volume64(U, B.dv[z], u);
         }
         double guess = 0.0;
         if (MLP && a.srhd) {
@@ -65,7 +64,7 @@ struct F64C2p {
                 iters += it2;
             }
         } else {
-            kind = newt_c2p(a.gm - 1.0, u, P, bad);
+            kind = newt_c2p64(a.gm - 1.0, u, P, bad);
         }
         ++st.zones;
         st.it64 += (unsigned)iters;
@@ -73,8 +72,7 @@ struct F64C2p {
             atomicMin(&a.status->err_key, error_key(a.stage, slot, i, j, kind));
             a.status->err_sel = a.sel_in;
         }
-        const double w = a.srhd ? sqrt(1.0 + P[1] * P[1] + P[2] * P[2]) : 1.0;
-        double v[NFIELD] = {P[0], P[1], P[2], P[3], smass / dV / w};
+        const double v[NFIELD] = {P[0], P[1], P[2], P[3], a.srhd ? over_lorentz64(u[4], P[1], P[2]) : u[4]};
         store_prim<double>(B, i, j, v);
         if (a.compute_dt) {
             PhysT<double> ph;
@@ -87,7 +85,7 @@ struct F64C2p {
             const double dr = B.rv[i + 1] - B.rv[i];
             const double dq = B.qv[j + 1] - B.qv[j];
             const double dl = fmin(dr, dq * B.rv[i]);
-            const double amax = max_signal_speed(ph, P) * a.cflux;
+            const double amax = max_signal_speed64(ph, P) * a.cflux;
             st.dtz = fmin(st.dtz, dl / amax);
         }
     }
@@ -310,26 +308,6 @@ cudaError_t launch_c2p_f64(const StageArgs& a, cudaStream_t s) {
     return cudaGetLastError();
 }
 
-template <int TR>
-static void update_f64(const StageArgs& a, cudaStream_t s) {
-    update_kernel<double, false, TR><<<a.nutiles, update_threads<TR>(), StageSmem<double, TR>::bytes, s>>>(a);
-}
-
-cudaError_t launch_update_f64(const StageArgs& a, cudaStream_t s) {
-    if (a.strips) {
-        if (a.nstrips <= 0) return cudaSuccess;
-        update_strip_kernel<double, false, 2><<<(a.nstrips + STRIP_WARPS - 1) / STRIP_WARPS, STRIP_WARPS * 32, 0, s>>>(a);
-        return cudaGetLastError();
-    }
-    if (a.nutiles <= 0) return cudaSuccess;
-    switch (a.utr) {
-    case 4: update_f64<4>(a, s); break;
-    case 16: update_f64<16>(a, s); break;
-    default: update_f64<8>(a, s);
-    }
-    return cudaGetLastError();
-}
-
 template <int TR, bool MLP>
 static cudaError_t fused_f64(const StageArgs& a, const GhostArgs& g, const FusedArgs& f, int grid, cudaStream_t s) {
     cudaLaunchConfig_t cfg = {};
@@ -375,17 +353,8 @@ static cudaError_t configure_fused_f64() {
                                 (int)fused_smem_bytes<double, TR, MLP>());
 }
 
-template <int TR>
-static cudaError_t configure_update_f64() {
-    return cudaFuncSetAttribute(update_kernel<double, false, TR>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                (int)StageSmem<double, TR>::bytes);
-}
-
 cudaError_t configure_f64() {
-    cudaError_t e = configure_update_f64<4>();
-    if (e == cudaSuccess) e = configure_update_f64<8>();
-    if (e == cudaSuccess) e = configure_update_f64<16>();
-    if (e == cudaSuccess) e = configure_fused_f64<4, false>();
+    cudaError_t e = configure_fused_f64<4, false>();
     if (e == cudaSuccess) e = configure_fused_f64<8, false>();
     if (e == cudaSuccess) e = configure_fused_f64<16, false>();
     if (e == cudaSuccess) e = configure_fused_f64<4, true>();

@@ -14,6 +14,7 @@
 #include "knc_internal.h"
 #include "knc_models.cuh"
 #include "knc_physics.cuh"
+#include "knc_physics64.cuh"
 
 namespace knc {
 
@@ -137,9 +138,9 @@ __device__ __forceinline__ void recover_hp(const double gm, const double (&U)[5]
         v[3] = p < 0.0 ? PRESSURE_FLOOR * v[0] : p / dv;
     } else {
         const double u[4] = {m, s1, s2, tau};
-        double Pd[4];
-        double bad;
-        if (srhd_c2p_newton(gm, u, 0.0, Pd, it, bad) == HYDRO_ROOT_FINDER_FAILED) return;
+        double Pd[4] = {0.0, 0.0, 0.0, 0.0};
+        double bad = 0.0;
+        if (srhd_c2p_plain(gm, u, 0.0, Pd, &it, &bad) == HYDRO_ROOT_FINDER_FAILED) return;
         v[0] = Pd[0] / dv;
         v[1] = Pd[1];
         v[2] = Pd[2];

@@ -114,7 +114,7 @@ struct StageArgs {
     const DevBlock* blocks;
     const int4* tiles;      // {slot, i0, j0, 0}, TILE_R x TILE_Q (recovery, init)
     int32_t ntiles;
-    const int4* utiles;     // {slot, i0, j0, 0}, utr x TILE_Q (update)
+    const int4* utiles;     // {slot, i0, j0, rows}, utr x TILE_Q (update)
     int32_t nutiles;
     int32_t utr;            // update tile rows: 4, 8 or 16
     int32_t tma;            // mixed update: stage tiles with tensor copies (tmaps valid)
@@ -249,6 +249,8 @@ void host_block_volumes(const knc_mesh_params& mesh, int32_t index, std::vector<
 cudaError_t configure_kernels();
 cudaError_t launch_init_f64(const InitArgs& a, int ntiles, cudaStream_t s);
 cudaError_t launch_c2p_f64(const StageArgs& a, cudaStream_t s);
+// The FP64 update over the items {slot, i0, j0, rows <= 32} of a.strips (or
+// a.utiles), 32 columns each (knc_f64_update.cu).
 cudaError_t launch_update_f64(const StageArgs& a, cudaStream_t s);
 cudaError_t launch_ghost_f64(const GhostArgs& a, cudaStream_t s);
 cudaError_t launch_ghost_mixed(const GhostArgs& a, cudaStream_t s);

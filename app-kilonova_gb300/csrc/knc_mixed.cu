@@ -93,7 +93,7 @@ __device__ __forceinline__ Fp64Recovery recover_fp64(const StageArgs& a, double 
         double Pd[4] = {0.0, 0.0, 0.0, 0.0};
         double bad;
         int itf = 0;
-        const int kf = srhd_c2p_newton(a.gm, u, 0.0, Pd, itf, bad);
+        const int kf = srhd_c2p_plain(a.gm, u, 0.0, Pd, &itf, &bad);
         r.it64 += itf;
         if (kf == HYDRO_ROOT_FINDER_FAILED) {
             r.kind = kf;

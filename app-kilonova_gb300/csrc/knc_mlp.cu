@@ -22,6 +22,7 @@
 #include "knc_internal.h"
 #include "knc_mlp.cuh"
 #include "knc_physics.cuh"
+#include "knc_physics64.cuh"
 #include "knc_tc.cuh"
 #include "knc_tma.cuh"
 

@@ -24,6 +24,7 @@
 
 #include "knc_internal.h"
 #include "knc_physics.cuh"
+#include "knc_physics64.cuh"
 
 namespace knc {
 

@@ -498,7 +498,7 @@ __device__ __forceinline__ R lorentz_factor(const PhysT<R>& ph, const R* P) {
 // X = tau + m (1 - W) + p (1 - W^2), rho h = m / W + rho e + p and
 // f / f' = f rho h / (v^2 gamma p - rho h). Returns HYDRO_* and the
 // iteration count.
-__device__ __forceinline__ int srhd_c2p_newton(double gm, const double* U, double guess, double* P,
+__device__ __forceinline__ int srhd_c2p_newton_plain(double gm, const double* U, double guess, double* P,
                                                int& iterations, double& bad) {
     const double m = U[0];
     const double tau = U[3];

@@ -10,6 +10,7 @@
 
 #include "../../include/knc.h"
 #include "knc_bits.cuh"
+#include "knc_fp64.cuh"
 
 namespace {
 
@@ -41,7 +42,40 @@ __global__ void conversions_kernel(const double* in, int64_t n, double* out) {
     out[4 * k + 3] = knc::half_exact(x);
 }
 
+__global__ void fp64_ops_kernel(const double* in, int64_t n, double* out) {
+    const int64_t k = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (k >= n) return;
+    const double a = in[2 * k], b = in[2 * k + 1], c = fabs(b);
+    const knc::Start64 y = knc::rcp_start(b), r = knc::rsqrt_start(c);
+    const double w = knc::fp64_sqrt(c, r);
+    out[6 * k + 0] = knc::fp64_div(a, b, y);
+    out[6 * k + 1] = knc::fp64_rcp(b, y);
+    out[6 * k + 2] = w;
+    out[6 * k + 3] = knc::fp64_div(a, w, r);
+    out[6 * k + 4] = knc::fp64_min(a, b);
+    out[6 * k + 5] = knc::fp64_max(a, b);
+}
+
 }  // namespace
+
+extern "C" int knc_test_fp64_ops(const double* in, int64_t n, double* out) {
+    if (!in || !out || n <= 0) return KNC_ERR_INVALID_ARGUMENT;
+    double *d_in = nullptr, *d_out = nullptr;
+    if (cudaMalloc(&d_in, n * 16) != cudaSuccess) return KNC_ERR_OUT_OF_MEMORY;
+    if (cudaMalloc(&d_out, n * 48) != cudaSuccess) {
+        cudaFree(d_in);
+        return KNC_ERR_OUT_OF_MEMORY;
+    }
+    cudaError_t e = cudaMemcpy(d_in, in, n * 16, cudaMemcpyHostToDevice);
+    if (e == cudaSuccess) {
+        fp64_ops_kernel<<<(unsigned)((n + 255) / 256), 256>>>(d_in, n, d_out);
+        e = cudaGetLastError();
+    }
+    if (e == cudaSuccess) e = cudaMemcpy(out, d_out, n * 48, cudaMemcpyDeviceToHost);
+    cudaFree(d_in);
+    cudaFree(d_out);
+    return e == cudaSuccess ? KNC_OK : KNC_ERR_CUDA;
+}
 
 extern "C" int knc_test_conversions(const double* in, int64_t n, double* out) {
     if (!in || !out || n <= 0) return KNC_ERR_INVALID_ARGUMENT;

@@ -471,6 +471,12 @@ int knc_recover_primitives_noalloc(const knc_hydro_params* hydro, const knc_mesh
  * hardware d2f, integer-pipe x / 2). */
 int knc_test_conversions(const double* in, int64_t n, double* out);
 
+/* Self-test of the FP64 stage's division, reciprocal, square root, minimum
+ * and maximum on the integer pipe: for n pairs (a, b) = in[2 * k + 0..1], with
+ * magnitudes in 2^[-400, 400] (a may be zero), writes
+ * out[6 * k + 0..5] = (a / b, 1 / b, sqrt|b|, a / sqrt|b|, min(a, b), max(a, b)). */
+int knc_test_fp64_ops(const double* in, int64_t n, double* out);
+
 /* Measured FP64 FMA throughput of the current device (GFLOP/s, 2/FMA). */
 int knc_measure_fp64_peak(double* gflops);
 
