@@ -2542,7 +2542,7 @@ int stream_step(knc_ctx* c, double dt, const double* hc_in, const double* hs_in,
                                     mixed(c) ? 4 : 8, st));
                 ++c->launches;
                 if (g[s].P64[end]) {
-                    // mixed: the rows in FP64 too (zone_hp reads those above the split)
+                    // mixed: the rows in FP64 too (zones_hp reads those above the split)
                     CK(launch_halo_rows(gscratch64(s, end), g[s].P64[end], g[s].nq[end], g[s].nr_t[end],
                                         g[s].row0[end], 8, st));
                     ++c->launches;

@@ -101,7 +101,7 @@ static __device__ __noinline__ void ghost_zone(const GhostArgs& a, int end, int 
         float* Pd = reinterpret_cast<float*>(a.P[end]);
 #pragma unroll
         for (int c = 0; c < NFIELD; ++c) Pd[c * pn + off] = (float)v[c];
-        // above the Lorentz-factor split: the FP64 row for zone_hp, and listed
+        // above the Lorentz-factor split: the FP64 row for zones_hp, and listed
         if (a.P64[end] && high_zone((float)v[1], (float)v[2], a.uu_high_f)) {
 #pragma unroll
             for (int c = 0; c < NFIELD; ++c) a.P64[end][c * pn + off] = v[c];

@@ -61,7 +61,7 @@ struct DevBlock {
     // mixed stage: FP64 primitives [5][nr+4][nq] like P, written only for the
     // zones whose stored FP32 primitive is above the Lorentz-factor split
     // (own rows by the recovery, halo rows by the neighbours' recovery, the
-    // ghost and the remap launches), read by zone_hp; null in the FP64 stage
+    // ghost and the remap launches), read by zones_hp; null in the FP64 stage
     double* P64;
     void* P_in_nbr;        // inner neighbour's P: my rows 0,1 go to its rows nr'+2, nr'+3
     void* P_out_nbr;       // outer neighbour's P: my rows nr-2, nr-1 go to its rows 0, 1
@@ -145,7 +145,7 @@ struct StageArgs {
     float high_thr_f;       // 1 - 1 / w_split^2: |S| / (D + tau) squared above it means W > w_split
     // mixed update: a zone whose stored FP32 four-velocity has
     // u_r^2 + u_theta^2 = W^2 - 1 above uu_high_f (W above the split) makes
-    // every face whose 4-zone stencil reaches it an FP64 face (zone_hp)
+    // every face whose 4-zone stencil reaches it an FP64 face (zones_hp)
     float uu_high_f;
     // mixed stage: every stored FP32 primitive above the Lorentz-factor split,
     // as {slot, padded row x nq + column} of the block whose P array holds it

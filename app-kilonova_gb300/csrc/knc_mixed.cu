@@ -8,7 +8,7 @@
 //         radius (host), and the cons -> prim recovery of zones whose Lorentz
 //         factor exceeds `w_split` — converged to the reference's residual
 //         |f| < 1e-12 (D + tau) — and the faces whose stencil reaches such a
-//         zone, with the update of the zones they bound (zone_hp,
+//         zone, with the update of the zones they bound (zones_hp,
 //         knc_stage.cuh).
 // Zones below `w_split` recover in FP32. Every zone first runs the Newton
 // iteration in FP32; an FP64 recovery then starts from that root and usually
@@ -661,7 +661,8 @@ static void update_mixed(const StageArgs& a, cudaStream_t s) {
 
 template <int MB>
 static void update_strips(const StageArgs& a, cudaStream_t s) {
-    const int want = (a.nstrips + STRIP_WARPS - 1) / STRIP_WARPS;
+    // (with a list at least one CTA per SM: its zones are claimed by every warp)
+    const int want = std::max((a.nstrips + STRIP_WARPS - 1) / STRIP_WARPS, a.hp_list ? num_sms() : 1);
     const int grid = std::min(want, resident_grid(update_strip_kernel<float, true, MB>, STRIP_WARPS * 32, 0));
     launch_chained(update_strip_kernel<float, true, MB>, grid, STRIP_WARPS * 32, 0, s, a);
 }

@@ -22,6 +22,7 @@
 #include "knc_bits.cuh"
 #include "knc_internal.h"
 #include "knc_physics.cuh"
+#include "knc_physics64.cuh"
 
 namespace knc {
 
@@ -108,7 +109,7 @@ __device__ __forceinline__ R stage_dt(const StageArgs& a) {
 // for the recovery: every face whose 4-zone stencil holds a zone with
 // W > w_split (judged from the stored FP32 four-velocity, the same test in
 // every update form) is solved in FP64 from FP64 primitives, and the zones
-// such faces bound are updated in FP64 (zone_hp, after the strip helpers).
+// such faces bound are updated in FP64 (zones_hp, after the strip helpers).
 
 // The FP64 faces of zone (i, j) from the relativistic zones of its plus-shaped
 // stencil: col bit k = zone (i - 2 + k, j), row bit k = zone (i, j - 2 + k),
@@ -119,7 +120,7 @@ __device__ __forceinline__ unsigned hp_faces(unsigned col, unsigned row) {
            ((row & 0x1eu) ? 8u : 0u);
 }
 
-static __device__ __noinline__ void zone_hp(const StageArgs& a, const DevBlock& B, int i, int j);
+__device__ __forceinline__ void row_zones_hp(const StageArgs& a, int slot, int i, int j0, unsigned m);
 __device__ __forceinline__ void drain_hp(const StageArgs& a);
 __device__ __forceinline__ void clear_next_hp(const StageArgs& a);
 
@@ -282,8 +283,9 @@ __device__ __forceinline__ void update_tile(const StageArgs& a, const int4 t, un
         const int i = i0 + r, j = j0 + c;
         unsigned hpf = 0u;
         if constexpr (MIXED) {
-            // FP64 faces (a relativistic zone in the plus stencil): zone_hp
-            if (i < nr && j < nq && stage_has_high(a)) {
+            // FP64 faces (a relativistic zone in the plus stencil): zones_hp
+            const bool some = stage_has_high(a);
+            if (i < nr && j < nq && some) {
                 unsigned cm = 0u, rm = 0u;
 #pragma unroll
                 for (int k = 0; k < 5; ++k) {
@@ -293,9 +295,11 @@ __device__ __forceinline__ void update_tile(const StageArgs& a, const int4 t, un
                     rm |= high_zone(zr[0], zr[PR * PQS], a.uu_high_f) ? 1u << k : 0u;
                 }
                 hpf = hp_faces(cm, rm);
-                // with a list the zone waits for drain_hp; without, it is updated here
-                if (hpf && !a.hp_list) zone_hp(a, B, i, j);
             }
+            // with a list the zone waits for drain_hp; without, it is updated
+            // here (a warp holds one row of the tile, lane = column)
+            if (some && !a.hp_list)
+                row_zones_hp(a, t.x, i, j0 + 2, __ballot_sync(0xffffffffu, hpf != 0u));
         }
         if (i < nr && j < nq && !(MIXED && hpf)) {
             const int64_t n = (int64_t)nr * nq;
@@ -422,7 +426,7 @@ __device__ __forceinline__ void strip_face(const PhysT<R>& ph, const StageArgs& 
     }
 }
 
-// ---- FP64 faces of the mixed stage at high Lorentz factor (zone_hp) -----------
+// ---- FP64 faces of the mixed stage at high Lorentz factor (zones_hp) ----------
 // FP64 primitive (rho, u_r, u_theta, p, s) of zone (r, c) of block B,
 // r in [-2, nr + 1] (padded rows, halo included): a zone above the split
 // takes the FP64 primitive its producer stored in P64 (the recovery from
@@ -443,134 +447,175 @@ __device__ __forceinline__ void prim_hp(const StageArgs& a, const DevBlock& B, i
     }
 }
 
-// One face from its stencil s[0..3] (the face between s[1] and s[2]) with the
-// stage's limiter; zl / zr: zero slope for s[1] / s[2] (the block's first and
-// last column). FP64: the reference's face solve. FP32: the instructions the
-// update forms run for the same face, so the value equals theirs.
-template <class R>
-__device__ __forceinline__ void face_states(R th, const R (*s)[NFIELD], bool zl, bool zr, R pl[NFIELD],
-                                            R pr[NFIELD]) {
+// Half slopes of one field over a stencil in the stage's limiter: FP64 in the
+// form of knc_physics64.cuh, FP32 with the update forms' instructions.
+__device__ __forceinline__ double hp_half_slope(double th, double a, double b, double c) {
+    return half_slope64(th * (b - a), c - a, th * (c - b));
+}
+
+// Flux x c x area through face f of zone (i, j) (0: radial i, 1: radial i + 1,
+// 2: polar j, 3: polar j + 1) from the stencil's four zones; `high`: some of
+// them is above the split, and the face is solved in FP64 from FP64
+// primitives (prim_hp); else again in FP32 with the update forms' own
+// instructions, so a face shared with a zone of the FP32 update carries the
+// same flux on both sides. Both zones of an FP64 face solve it from the same
+// inputs with the same instructions.
+__device__ __forceinline__ void hp_face(const StageArgs& a, const DevBlock& B, int i, int j, int f, bool high,
+                                        double (&F)[NFIELD]) {
+    const int nq = B.nq, nr = B.nr;
+    const bool radial = f < 2;
+    const int k = radial ? i + f : j + (f - 2);   // between rows / columns k - 1 and k
+    const bool exists = radial ? k <= nr : (k > 0 && k < nq && i < nr);
+    const bool zl = !radial && (k - 1 == 0 || k - 1 == nq - 1);   // zero polar slope on the edge columns
+    const bool zr = !radial && (k == 0 || k == nq - 1);
 #pragma unroll
-    for (int q = 0; q < NFIELD; ++q) {
-        const R gl = zl ? R(0) : stage_plm<R, sizeof(R) == 4>(th, s[0][q], s[1][q], s[2][q]);
-        const R gr = zr ? R(0) : stage_plm<R, sizeof(R) == 4>(th, s[1][q], s[2][q], s[3][q]);
-        pl[q] = s[1][q] + gl * R(0.5);
-        pr[q] = s[2][q] - gr * R(0.5);
+    for (int q = 0; q < NFIELD; ++q) F[q] = 0.0;
+    if (!exists) return;
+    if (high) {
+        const PhysT<double> ph = make_phys<double>(a);
+        double s[4][NFIELD];
+#pragma unroll
+        for (int m = 0; m < 4; ++m) {
+            const int r = radial ? k - 2 + m : i, c = radial ? j : k - 2 + m;
+            if (radial || (c >= 0 && c < nq)) {
+                prim_hp(a, B, r, c, s[m]);
+            } else {
+#pragma unroll
+                for (int q = 0; q < NFIELD; ++q) s[m][q] = 0.0;
+            }
+        }
+        double pl[NFIELD], pr[NFIELD], out[NFIELD];
+#pragma unroll
+        for (int q = 0; q < NFIELD; ++q) {
+            pl[q] = s[1][q] + (zl ? 0.0 : hp_half_slope(ph.theta, s[0][q], s[1][q], s[2][q]));
+            pr[q] = s[2][q] - (zr ? 0.0 : hp_half_slope(ph.theta, s[1][q], s[2][q], s[3][q]));
+        }
+        if (a.hllc) face64<true, true>(ph, a.gm_f, a.gh_f, pl, pr, radial ? 0 : 1, out);
+        else face64<true, false>(ph, a.gm_f, a.gh_f, pl, pr, radial ? 0 : 1, out);
+        const double A = radial ? B.ar[(int64_t)k * nq + j] : B.aq[(int64_t)i * (nq + 1) + k];
+#pragma unroll
+        for (int q = 0; q < NFIELD; ++q) F[q] = out[q] * a.cflux * A;
+    } else {
+        const PhysT<float> ph = make_phys<float>(a);
+        const float* P = reinterpret_cast<const float*>(B.P);
+        const int64_t pn = (int64_t)(nr + 4) * nq;
+        float s[4][NFIELD];
+#pragma unroll
+        for (int m = 0; m < 4; ++m) {
+            const int c = radial ? j : k - 2 + m;
+            load_prim_row(P, pn, nq, nr, c, c >= 0 && c < nq, radial ? k - 2 + m : i, s[m]);
+        }
+        float pl[NFIELD], pr[NFIELD], out[NFIELD] = {0.f, 0.f, 0.f, 0.f, 0.f};
+#pragma unroll
+        for (int q = 0; q < NFIELD; ++q) {
+            const float gl = zl ? 0.f : plm_gradient_f32(ph.theta, s[0][q], s[1][q], s[2][q]);
+            const float gr = zr ? 0.f : plm_gradient_f32(ph.theta, s[1][q], s[2][q], s[3][q]);
+            pl[q] = s[1][q] + gl * 0.5f;
+            pr[q] = s[2][q] - gr * 0.5f;
+        }
+        strip_face<float, true>(ph, a, B, radial ? 0 : 1, pl, pr, radial ? k : i, radial ? j : k, nq, a.cflux_f, out);
+        // FP32 fluxes carry areas in the stage's length units
+        const double l2 = words((uint32_t)(1023 + a.lscale2) << 20, 0u);
+#pragma unroll
+        for (int q = 0; q < NFIELD; ++q) F[q] = (double)out[q] * l2;
     }
 }
 
-// Zone (i, j) of the mixed stage when its plus-shaped stencil holds a zone
-// above the Lorentz-factor split (update forms: high_zone / hp_faces). Its
-// faces whose 4-zone stencil holds such a zone are solved in FP64 from FP64
-// primitives (prim_hp); its other faces are solved again in FP32 from the
-// stored primitives with the update forms' own instructions, so a face
-// shared with a zone of the FP32 update carries the same flux on both sides.
-// Sources, update and RK average in FP64, written to U_out. Every zone
-// bordering an FP64 face solves that face from the same inputs with the same
-// instructions, so both of its zones see one flux.
-static __device__ __noinline__ void zone_hp(const StageArgs& a, const DevBlock& B, int i, int j) {
+// Which faces of zone (i, j) are FP64 faces (hp_faces), from the stored FP32
+// four-velocities of its plus-shaped stencil (zero outside the padded rows
+// and the block's columns).
+__device__ __forceinline__ unsigned zone_hp_faces(const StageArgs& a, const DevBlock& B, int i, int j) {
     const int nq = B.nq, nr = B.nr;
-    const float* P = reinterpret_cast<const float*>(B.P);
     const int64_t pn = (int64_t)(nr + 4) * nq;
-    // FP32 primitives as the update forms see them: col32[k] zone (i - 2 + k, j),
-    // row32[k] zone (i, j - 2 + k), zero outside the padded rows and the block's columns
-    float col32[5][NFIELD], row32[5][NFIELD];
+    const float* Pu = reinterpret_cast<const float*>(B.P) + pn;   // u_r; u_theta one field on
     unsigned cm = 0u, rm = 0u;
+#pragma unroll
     for (int k = 0; k < 5; ++k) {
-        const int c = j - 2 + k;
-        load_prim_row(P, pn, nq, nr, j, true, i - 2 + k, col32[k]);
-        load_prim_row(P, pn, nq, nr, c, c >= 0 && c < nq, i, row32[k]);
-        cm |= high_zone(col32[k][1], col32[k][2], a.uu_high_f) ? 1u << k : 0u;
-        rm |= high_zone(row32[k][1], row32[k][2], a.uu_high_f) ? 1u << k : 0u;
+        const bool rok = i + k < nr + 4, cok = j - 2 + k >= 0 && j - 2 + k < nq;
+        const int64_t ro = rok ? (int64_t)(i + k) * nq + j : 0, co = cok ? (int64_t)(i + 2) * nq + j - 2 + k : 0;
+        cm |= rok && high_zone(Pu[ro], Pu[pn + ro], a.uu_high_f) ? 1u << k : 0u;
+        rm |= cok && high_zone(Pu[co], Pu[pn + co], a.uu_high_f) ? 1u << k : 0u;
     }
-    const unsigned faces = hp_faces(cm, rm);
-    const PhysT<float> ph32 = make_phys<float>(a);
-    const PhysT<double> ph = make_phys<double>(a);
-    // col[k]: zone (i - 2 + k, j); row[k]: zone (i, j - 2 + k), FP64
-    double col[5][NFIELD], row[5][NFIELD];
-    prim_hp(a, B, i, j, col[2]);
+    return hp_faces(cm, rm);
+}
+
+// Eight zones of the mixed stage with FP64 faces (a zone above the Lorentz-factor
+// split in the plus-shaped stencil), four lanes to a zone: lane f of a zone's
+// four solves its face f, then the lanes share the zone's update (component
+// f; lane 0 the scalar too): sources, update and RK average in FP64, written
+// to U_out. FP64 instructions cost the same however many lanes are active, so
+// a zone on one lane, its faces one after the other, left the pipe 4 times
+// longer at work. Every lane of the warp calls it; lanes whose zone is not
+// active only take part in the exchange.
+static __device__ __noinline__ void zones_hp(const StageArgs& a, int slot, int i, int j, bool active) {
+    const unsigned full = 0xffffffffu;
+    const int f = threadIdx.x & 3;
+    const DevBlock& B = a.blocks[slot];
+    double F[NFIELD] = {0.0, 0.0, 0.0, 0.0, 0.0};
+    if (active) hp_face(a, B, i, j, f, (zone_hp_faces(a, B, i, j) >> f) & 1u, F);
+    __syncwarp(full);
+    // dr = F(1) - F(0), dq = F(3) - F(2) of component f on lane f (and of the
+    // scalar): the faces' fluxes by shuffles within the four lanes
+    double dr = 0.0, dq = 0.0, dr4 = 0.0, dq4 = 0.0;
+    const int base = threadIdx.x & 28;
 #pragma unroll
-    for (int q = 0; q < NFIELD; ++q) row[2][q] = col[2][q];
-    if (faces & 3u)
-        for (int k = 0; k < 5; ++k)
-            if (k != 2) prim_hp(a, B, i - 2 + k, j, col[k]);
-    if (faces & 12u)
-        for (int k = 0; k < 5; ++k) {
-            const int c = j - 2 + k;
-            if (k == 2) continue;
-            if (c >= 0 && c < nq) {
-                prim_hp(a, B, i, c, row[k]);
-            } else {
-#pragma unroll
-                for (int q = 0; q < NFIELD; ++q) row[k][q] = 0.0;
-            }
+    for (int q = 0; q < NFIELD; ++q) {
+        const double f0 = __shfl_sync(full, F[q], base), f1 = __shfl_sync(full, F[q], base + 1);
+        const double f2 = __shfl_sync(full, F[q], base + 2), f3 = __shfl_sync(full, F[q], base + 3);
+        if (q == f) {
+            dr = __dsub_rn(f1, f0);
+            dq = __dsub_rn(f3, f2);
         }
-    const double l2 = ldexp(1.0, a.lscale2);   // FP32 fluxes carry areas in the stage's length units
-    double F[4][NFIELD];
-    for (int f = 0; f < 4; ++f) {
-        // face f: radial i, radial i + 1, polar j, polar j + 1
-        const bool radial = f < 2;
-        const int k = radial ? i + f : j + (f - 2);   // between rows / columns k - 1 and k
-        const bool exists = radial ? k <= nr : (k > 0 && k < nq && i < nr);
-        const bool zl = !radial && (k - 1 == 0 || k - 1 == nq - 1);
-        const bool zr = !radial && (k == 0 || k == nq - 1);
-#pragma unroll
-        for (int q = 0; q < NFIELD; ++q) F[f][q] = 0.0;
-        if (!exists) continue;
-        if ((faces >> f) & 1u) {
-            double pl[NFIELD], pr[NFIELD], out[NFIELD];
-            face_states<double>(ph.theta, radial ? &col[f] : &row[f - 2], zl, zr, pl, pr);
-            riemann(ph, pl, pr, pl[4], pr[4], radial ? 0 : 1, out);
-            const double A = radial ? B.ar[(int64_t)k * nq + j] : B.aq[(int64_t)i * (nq + 1) + k];
-#pragma unroll
-            for (int q = 0; q < NFIELD; ++q) F[f][q] = out[q] * a.cflux * A;
-        } else {
-            float pl[NFIELD], pr[NFIELD], out[NFIELD] = {0.f, 0.f, 0.f, 0.f, 0.f};
-            face_states<float>(ph32.theta, radial ? &col32[f] : &row32[f - 2], zl, zr, pl, pr);
-            strip_face<float, true>(ph32, a, B, radial ? 0 : 1, pl, pr, radial ? k : i, radial ? j : k, nq,
-                                    a.cflux_f, out);
-#pragma unroll
-            for (int q = 0; q < NFIELD; ++q) F[f][q] = (double)out[q] * l2;
+        if (q == 4 && f == 0) {
+            dr4 = __dsub_rn(f1, f0);
+            dq4 = __dsub_rn(f3, f2);
         }
     }
-    const int64_t n = (int64_t)nr * nq, z = (int64_t)i * nq + j;
-    double src[4];
-    sources(ph, col[2], B.rc[i], B.cot[j], src);
-    const double dv = B.dv[z];
+    if (!active) return;
+    const int nq = B.nq;
+    const int64_t n = (int64_t)B.nr * nq, z = (int64_t)i * nq + j;
     const double dt = stage_dt<double>(a);
     const double* Uin = B.buf[a.sel_in];
     double* Uout = B.buf[a.sel_out];
-    double res[NFIELD];
-#pragma unroll
-    for (int q = 0; q < 4; ++q) {
-        const double du = (src[q] * a.cflux * dv - (F[1][q] - F[0][q]) - (F[3][q] - F[2][q])) * dt;
-        res[q] = Uin[q * n + z] + du;
+    const double* U0 = a.sel_base >= 0 ? B.buf[a.sel_base] : nullptr;
+    auto average = [&](double res, int q) {
+        if (!U0) return res;
+        if (a.avg_half) return half_exact(__dadd_rn(res, U0[q * n + z]));
+        return __dadd_rn(__dmul_rn(res, a.w1), __dmul_rn(U0[q * n + z], a.bf));
+    };
+    double src = 0.0;
+    if (f == 1 || f == 2) {
+        double P[NFIELD], s1, s2;
+        prim_hp(a, B, i, j, P);
+        sources64<true>(make_phys<double>(a), P, B.rc[i], B.cot[j], s1, s2);
+        src = (f == 1 ? s1 : s2) * a.cflux * B.dv[z];
     }
-    res[4] = Uin[4 * n + z] + ((F[1][4] - F[0][4]) + (F[3][4] - F[2][4])) * -dt;
-    if (a.sel_base >= 0) {
-        const double* U0 = B.buf[a.sel_base];
-        if (a.avg_half) {
-#pragma unroll
-            for (int q = 0; q < NFIELD; ++q) res[q] = half_exact(res[q] + U0[q * n + z]);
-        } else {
-#pragma unroll
-            for (int q = 0; q < NFIELD; ++q) res[q] = res[q] * a.w1 + U0[q * n + z] * a.bf;
-        }
+    Uout[f * n + z] = average(Uin[f * n + z] + (src - dr - dq) * dt, f);
+    if (f == 0) Uout[4 * n + z] = average(Uin[4 * n + z] + (dr4 + dq4) * -dt, 4);
+}
+
+// The zones (i, j0 - 2 + lane) of a row whose lanes are set in `m`, eight at a
+// time (stages without a list).
+__device__ __forceinline__ void row_zones_hp(const StageArgs& a, int slot, int i, int j0, unsigned m) {
+    const int k = (threadIdx.x & 31) >> 2;
+    while (m) {
+        unsigned t = m;
+        for (int q = 0; q < k; ++q) t &= t - 1u;   // drop the zones of the lower lanes
+        const bool active = t != 0u;
+        zones_hp(a, slot, i, j0 - 2 + (active ? __ffs(t) - 1 : 0), active);
+        for (int q = 0; q < 8; ++q) m &= m - 1u;
     }
-#pragma unroll
-    for (int q = 0; q < NFIELD; ++q) Uout[q * n + z] = res[q];
 }
 
 // ---- the zones with FP64 faces, from the stage's list of zones above the split
 // Work item c of listed zone h = (slot, padded row, column): the candidate
 // zone at offset c of h's plus-shaped neighbourhood (c < 5: rows -2..2 of
 // h's column; c >= 5: columns -2, -1, 1, 2 of h's row). A candidate inside
-// its block is updated by zone_hp if h is the first zone above the split in
-// the candidate's own plus stencil (column zones top to bottom, then row
-// zones left to right): every zone with FP64 faces has exactly one such
-// first zone, and every stored zone above the split is listed, so each is
-// updated once.
-__device__ __forceinline__ void hp_candidate(const StageArgs& a, unsigned item, unsigned c) {
+// its block is taken if h is the first zone above the split in the candidate's
+// own plus stencil (column zones top to bottom, then row zones left to
+// right): every zone with FP64 faces has exactly one such first zone, and
+// every stored zone above the split is listed, so each is updated once.
+__device__ __forceinline__ bool hp_candidate(const StageArgs& a, unsigned item, unsigned c, int4& zone) {
     const int2 e = a.hp_list[item];
     const DevBlock& B = a.blocks[e.x];
     const int nq = B.nq, nr = B.nr;
@@ -578,45 +623,67 @@ __device__ __forceinline__ void hp_candidate(const StageArgs& a, unsigned item, 
     const int d = (int)c < 5 ? (int)c - 2 : ((int)c < 7 ? (int)c - 7 : (int)c - 6);
     const int ic = (int)c < 5 ? ih + d : ih;
     const int jc = (int)c < 5 ? jh : jh + d;
-    if (ic < 0 || ic >= nr || jc < 0 || jc >= nq) return;
+    if (ic < 0 || ic >= nr || jc < 0 || jc >= nq) return false;
     const float* Pu = reinterpret_cast<const float*>(B.P) + (int64_t)(nr + 4) * nq;   // u_r; u_theta one field on
     const int64_t pn = (int64_t)(nr + 4) * nq;
-    auto high = [&](int i, int j) {
-        if (j < 0 || j >= nq) return false;
-        const int64_t off = (int64_t)(i + 2) * nq + j;
-        return high_zone(Pu[off], Pu[pn + off], a.uu_high_f);
-    };
-    int fi = 0, fj = -1;
-    for (int k = 0; k < 5 && fj < 0; ++k)
-        if (high(ic - 2 + k, jc)) {
-            fi = ic - 2 + k;
-            fj = jc;
-        }
-    for (int k = 0; k < 5 && fj < 0; ++k)
-        if (k != 2 && high(ic, jc - 2 + k)) {
-            fi = ic;
-            fj = jc - 2 + k;
-        }
-    if (fi == ih && fj == jh) zone_hp(a, B, ic, jc);
+    // one bit per zone of the stencil in that order (all loads in flight at once)
+    unsigned bits = 0u, mine = 0u;
+#pragma unroll
+    for (int k = 0; k < 9; ++k) {
+        const int i = k < 5 ? ic - 2 + k : ic, j = k < 5 ? jc : jc + (k < 7 ? k - 7 : k - 6);
+        const bool in = j >= 0 && j < nq;
+        const int64_t off = (int64_t)(i + 2) * nq + (in ? j : jc);
+        bits |= in && high_zone(Pu[off], Pu[pn + off], a.uu_high_f) ? 1u << k : 0u;
+        if (i == ih && j == jh) mine |= 1u << k;
+    }
+    zone = make_int4(e.x, ic, jc, 0);
+    return bits != 0u && (mine & (bits & (0u - bits))) != 0u;
 }
 
-// The update's second part: whole warps claim 32 work items at a time until
-// the list's 9 items per listed zone are done. The list is complete before
-// the update starts (the recovery, ghost and remap launches wrote it), and
-// the zones it updates are the ones every update form left untouched.
+// The update's second part: warps claim 32 work items at a time until the
+// list's 9 items per listed zone are done, and update the taken zones eight
+// at a time (about one item in nine is one): the zones a warp has taken wait
+// in its lanes 0..7. The list is complete before the update starts (the
+// recovery, ghost and remap launches wrote it), and the zones it updates are
+// the ones every update form left untouched.
 __device__ __forceinline__ void drain_hp(const StageArgs& a) {
     if (!a.hp_list) return;
     const unsigned count = min(*(volatile const unsigned*)a.hp_count, a.hp_cap);
     if (count == 0u) return;
+    const unsigned full = 0xffffffffu;
     const unsigned total = 9u * count;
-    const unsigned lane = threadIdx.x & 31u;
-    for (;;) {
-        unsigned base = 0u;
-        if (lane == 0u) base = atomicAdd(a.hp_claim, 32u);
-        base = __shfl_sync(0xffffffffu, base, 0);
-        if (base >= total) break;
-        const unsigned w = base + lane;
-        if (w < total) hp_candidate(a, w / 9u, w % 9u);
+    const int lane = threadIdx.x & 31;
+    int wait_slot = 0, wait_i = 0, wait_j = 0, n = 0;
+    bool more = true;
+    while (more || n > 0) {
+        unsigned mask = 0u;
+        int4 zone = make_int4(0, 0, 0, 0);
+        if (more) {
+            unsigned base = 0u;
+            if (lane == 0) base = atomicAdd(a.hp_claim, 32u);
+            base = __shfl_sync(full, base, 0);
+            more = base < total;
+            const unsigned w = base + (unsigned)lane;
+            mask = __ballot_sync(full, w < total && hp_candidate(a, w / 9u, w % 9u, zone));
+        }
+        do {
+            for (; mask && n < 8; ++n, mask &= mask - 1u) {
+                const int from = __ffs(mask) - 1;
+                const int s = __shfl_sync(full, zone.x, from), i = __shfl_sync(full, zone.y, from);
+                const int j = __shfl_sync(full, zone.z, from);
+                if (lane == n) {
+                    wait_slot = s;
+                    wait_i = i;
+                    wait_j = j;
+                }
+            }
+            if (n == 8 || (!more && n > 0)) {
+                const int k = lane >> 2, from = k < n ? k : 0;
+                zones_hp(a, __shfl_sync(full, wait_slot, from), __shfl_sync(full, wait_i, from),
+                         __shfl_sync(full, wait_j, from), k < n);
+                n = 0;
+            }
+        } while (mask);
     }
 }
 
@@ -671,7 +738,7 @@ __device__ __forceinline__ void update_strip(const StageArgs& a, const int4 it, 
         if (i0 <= nr && j < nq && jin) strip_face<R, MIXED>(ph, a, B, 0, pl, pr, i0, j, nq, cflux, Flo);
     }
     // mixed: hk = the warp's relativistic zones of window row i - 2 + k (bit =
-    // lane), warp-uniform; hp: some lane left zones to zone_hp
+    // lane), warp-uniform; hp: some lane left zones to zones_hp
     unsigned h0 = 0u, h1 = 0u, h2 = 0u, h3 = 0u, h4 = 0u;
     bool hp = false;
     if constexpr (HP) {
@@ -726,7 +793,7 @@ __device__ __forceinline__ void update_strip(const StageArgs& a, const int4 it, 
         }
         if (i + 1 <= nr && jin) strip_face<R, MIXED>(ph, a, B, 0, plr, prr, i + 1, j, nq, cflux, Fhi);
         // ---- mixed: a relativistic zone in the plus stencil (FP64 faces) leaves
-        // the zone to zone_hp after the row loop, its state untouched until then
+        // the zone to zones_hp after the row loop, its state untouched until then
         unsigned hpf = 0u;
         if constexpr (HP) {
             if ((h0 | h1 | h2 | h3 | h4) != 0u) {
@@ -807,8 +874,8 @@ __device__ __forceinline__ void update_strip(const StageArgs& a, const int4 it, 
             for (int s = 0; s < rows; ++s) {
                 h |= high_row(i0 + s + 2) << 4;
                 const unsigned m = __ballot_sync(full, (h & 4u) != 0u);
-                if (writes && hp_faces(h & 0x1fu, lane >= 2 ? (m >> (lane - 2)) & 0x1fu : 0u))
-                    zone_hp(a, B, i0 + s, jc);
+                const bool take = writes && hp_faces(h & 0x1fu, lane >= 2 ? (m >> (lane - 2)) & 0x1fu : 0u);
+                row_zones_hp(a, it.x, i0 + s, j0, __ballot_sync(full, take));
                 h >>= 1;
             }
         }
@@ -835,7 +902,7 @@ __device__ __forceinline__ bool strip_reaches_high(const StageArgs& a, const int
     return __any_sync(0xffffffffu, any);
 }
 
-// A strip with FP64 faces, out of line: its detection and zone_hp calls stay
+// A strip with FP64 faces, out of line: its detection and zones_hp calls stay
 // out of the register allocation of the common strip.
 static __device__ __noinline__ void update_strip_hp(const StageArgs& a, const int4 it) {
     update_strip<float, true, true>(a, it, make_phys<float>(a));
