@@ -92,7 +92,7 @@ struct F64C2p {
 };
 
 template <bool MLP>
-__global__ void __launch_bounds__(TILE_THREADS) c2p_f64_kernel(StageArgs a) {
+__global__ void __launch_bounds__(TILE_THREADS, MLP ? 1 : 4) c2p_f64_kernel(StageArgs a) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     const unsigned long long ek = *(volatile unsigned long long*)&a.status->err_key;
     if (ek != NO_ERROR && (uint32_t)(ek >> 48) < (uint32_t)a.stage) return;
