@@ -2189,12 +2189,18 @@ int advance_impl(knc_ctx* c, int32_t fold, const double* dt_given) {
 namespace {
 
 // Chunks of consecutive slots for the host-state advance, about equal in
-// zones, at most HOST_CHUNKS and at least one slot each: bounds[k] ..
-// bounds[k + 1] - 1 are chunk k's slots. Fewer chunks start the downloads
-// later, more pay more per copy and per launch chain; measured on the
-// 4096 x 1024 wind (64 blocks), ms per step: 8 chunks 1.38, 10 1.35, 12
-// 1.39, 16 1.40, 24 1.45.
-constexpr int HOST_CHUNKS = 10;
+// zones, at least one slot each: bounds[k] .. bounds[k + 1] - 1 are chunk k's
+// slots. Fewer chunks start the downloads later, more pay more per copy and
+// per launch chain. Mixed stage, 4096 x 1024 wind (64 blocks), ms per step: 8
+// chunks 1.38, 10 1.35, 12 1.39, 16 1.40, 24 1.45. The FP64 stage computes
+// longer than it copies, and the ends of its kernels on small chunks cost
+// more than the copies they would hide: 10 chunks 7.81, 4 7.43, 3 7.34, 2 7.90,
+// 1 9.07. A chunk holds at least HOST_CHUNK_ZONES zones: the host issues a
+// chunk's copies, events and launches in about 16 us, the time the link takes
+// for so many (256 x 128 FP64 step: 4 chunks 303, 2 250, 1 240 us).
+constexpr int HOST_CHUNKS_MIXED = 10;
+constexpr int HOST_CHUNKS_F64 = 3;
+constexpr int64_t HOST_CHUNK_ZONES = 65536;
 // streams the chunks' launches are spread over (chunk k on k % HOST_STREAMS;
 // at 10 chunks 1, 2, 3, 4 streams measured 1.36, 1.35, 1.35, 1.35 ms; at 16
 // chunks 4 and 8 streams 1.40 and 1.42)
@@ -2203,11 +2209,11 @@ constexpr int HOST_STREAMS = 4;
 // chunks 1 and 2 measured 1.36 and 1.35 ms; at 16 chunks 2 and 4 both 1.40)
 constexpr int HOST_UPLOADS_AHEAD = 2;
 
-std::vector<int> chunk_bounds(const Layout& l) {
+std::vector<int> chunk_bounds(const Layout& l, int most) {
     const int nb = (int)l.slot_index.size();
-    const int G = std::min(HOST_CHUNKS, nb);
-    std::vector<int> b{0};
     const int64_t total = l.zone_off[nb];
+    const int G = (int)std::max<int64_t>(1, std::min<int64_t>(std::min(most, nb), total / HOST_CHUNK_ZONES));
+    std::vector<int> b{0};
     for (int g = 1; g < G; ++g) {
         const int64_t target = total * g / G;
         int s = b.back() + 1;
@@ -2220,8 +2226,8 @@ std::vector<int> chunk_bounds(const Layout& l) {
 
 // Whether every chunk boundary whose blocks exchange halo rows has the 2S
 // rows on both sides that its shadow blocks copy (S stages per step).
-bool chunks_fit(const Layout& l, int S) {
-    const std::vector<int> cb = chunk_bounds(l);
+bool chunks_fit(const Layout& l, int S, int most) {
+    const std::vector<int> cb = chunk_bounds(l, most);
     for (size_t k = 1; k + 1 < cb.size(); ++k) {
         const DevBlock& lo = l.tab_h[cb[k] - 1];
         const DevBlock& hi = l.tab_h[cb[k]];
@@ -2229,6 +2235,8 @@ bool chunks_fit(const Layout& l, int S) {
     }
     return true;
 }
+
+int most_chunks(const knc_ctx* c) { return mixed(c) ? HOST_CHUNKS_MIXED : HOST_CHUNKS_F64; }
 
 // Independent chunks for the host-state advance (S stages per step). Each
 // chunk boundary whose blocks exchange halo rows gets two shadow blocks of 2S
@@ -2249,7 +2257,7 @@ int build_chunks(knc_ctx* c, int S) {
     if (l.sc_S == S) return KNC_OK;
     l.sc_S = 0;
     const int nb = (int)l.slot_index.size();
-    l.sc_cb = chunk_bounds(l);
+    l.sc_cb = chunk_bounds(l, most_chunks(c));
     const std::vector<int>& cb = l.sc_cb;
     const int G = (int)cb.size() - 1;
     std::vector<DevBlock> tab = l.tab_h;
@@ -2621,7 +2629,7 @@ int knc_advance_host(knc_ctx* c, const double* cons_in, const double* scalar_in,
     // (the chunks update as warp strips, which need a polar grid)
     const bool streamed = pinned && fold > 0 && !adaptive && !c->fused && L(c).nremap == 0 &&
                           c->model.kind != KNC_MODEL_HOST && c->mesh.p.num_polar_zones > 1 &&
-                          chunks_fit(L(c), c->hp.runge_kutta_order);
+                          chunks_fit(L(c), c->hp.runge_kutta_order, most_chunks(c));
     if (!streamed) {
         // whole-state copies around the fold
         if ((r = knc_set_state(c, cons_in, scalar_in))) return r;

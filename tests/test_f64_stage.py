@@ -69,3 +69,32 @@ def test_update_items_match_oracle(flow, nr, nq, order):
     o.advance(1)
     assert np.array_equal(cons.array, np.concatenate([c.reshape(-1, 4) for _, (c, _) in sorted(o.state().items())]))
     assert np.array_equal(scal.array, np.concatenate([s.reshape(-1) for _, (_, s) in sorted(o.state().items())]))
+
+
+@pytest.mark.parametrize("precision", ["f64", "mixed"])
+@pytest.mark.parametrize("order", ["RK2", "RK3"])
+def test_host_state_chunks_on_a_larger_grid(precision, order):
+    """Grids large enough to be split into chunks: the host-state step equals
+    upload, advance and download."""
+    import knc
+    from knc import workloads
+    from knc.solver import PinnedArray
+    w = workloads.wind_small()
+    w.mesh.block_size = 11
+    w.mesh.num_radial_zones = 460
+    w.mesh.outer_radius = 2.0
+    w.mesh.num_polar_zones = 1010
+    w.hydro.runge_kutta_order = order
+    mode = knc.abi.KNC_PRECISION_MIXED if precision == "mixed" else knc.abi.KNC_PRECISION_FP64
+    s = knc.build_solver(w, precision=mode)
+    n = w.zones
+    assert n >= 4 * 65536
+    ci, si, co, so = (PinnedArray(k) for k in ((n, 4), (n,), (n, 4), (n,)))
+    s.get_state(ci.array, si.array)
+    s.advance_host(ci.array, si.array, 1, co.array, so.array)
+    want_c, want_s = np.empty((n, 4)), np.empty(n)
+    s.set_state(ci.array, si.array)
+    s.advance(1)
+    s.get_state(want_c, want_s)
+    assert np.array_equal(co.array, want_c) and np.array_equal(so.array, want_s)
+    assert not np.array_equal(co.array, ci.array)
