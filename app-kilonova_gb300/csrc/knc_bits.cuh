@@ -57,17 +57,15 @@ __device__ __forceinline__ double f2d(float x) {
 __device__ __forceinline__ float d2f_rn_exp(double x, int de) {
     const unsigned long long b = (unsigned long long)__double_as_longlong(x);
     const uint32_t hi = (uint32_t)(b >> 32), lo = (uint32_t)b;
-    const uint32_t sign = hi & 0x80000000u;
-    const uint32_t ex = (hi >> 20) & 0x7ffu;
-    const int e32 = (int)ex - 1023 + 127 + (ex ? de : 0);
-    const uint32_t m23 = ((hi & 0xfffffu) << 3) | (lo >> 29);
-    const uint32_t rest = lo & 0x1fffffffu;
-    uint32_t r = ((uint32_t)e32 << 23) + m23;
-    r += (rest > 0x10000000u) || (rest == 0x10000000u && (m23 & 1u));
-    r = e32 <= 0 ? 0u : r;
-    r = (e32 >= 255 || ex == 0x7ffu) ? 0x7f800000u : r;
-    r = r > 0x7f800000u ? 0x7f800000u : r;
-    return __uint_as_float(sign | r);
+    // exponent rebased in its field (below 1 << 20: under float's normal
+    // range, from 255 << 20: above it), then the upper 23 mantissa bits
+    const int32_t h = (int32_t)((hi & 0x7fffffffu) - ((uint32_t)(896 - de) << 20));
+    uint32_t r = __funnelshift_l(lo, (uint32_t)h, 3);
+    // the 29 dropped bits above one half, or one half and r odd
+    r += ((lo << 3) | (r & 1u)) > 0x80000000u ? 1u : 0u;
+    r = h < (1 << 20) ? 0u : r;
+    r = h >= (255 << 20) ? 0x7f800000u : r;
+    return __uint_as_float((hi & 0x80000000u) | r);
 }
 
 __device__ __forceinline__ double f2d_exp(float x, int de) {

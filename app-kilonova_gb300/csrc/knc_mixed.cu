@@ -155,7 +155,7 @@ struct MixedRemapRecovery {
         const float im = 1.0f / mf;
         const float s1n = s1f * im, s2n = s2f * im, taun = tauf * im;
         const float ssn = s1n * s1n + s2n * s2n;
-        const float x1 = __fdividef(sqrtf(ssn), 1.0f + taun);
+        const float x1 = __fdividef(sqrt_n(ssn), 1.0f + taun);
         const bool high = x1 * x1 > a.high_thr_f;
         float p32 = 0.f, w32 = 1.f;
         int it32 = 0;
@@ -163,9 +163,9 @@ struct MixedRemapRecovery {
         float P[4];
         int kind = HYDRO_NONE;
         if (!high && ok32) {
-            const float inv_dv = 1.0f / dV;
-            const float inv_et = 1.0f / (taun + 1.0f + p32);
-            P[0] = mf / w32 * inv_dv;
+            const float inv_dv = rcp_n(dV);
+            const float inv_et = rcp_n(taun + 1.0f + p32);
+            P[0] = mf * rcp_n(w32) * inv_dv;
             P[1] = w32 * s1n * inv_et;
             P[2] = w32 * s2n * inv_et;
             P[3] = p32 * mf * inv_dv;
@@ -176,10 +176,10 @@ struct MixedRemapRecovery {
             for (int q = 0; q < 4; ++q) P[q] = r.P[q];
             kind = r.kind;
         }
-        const float wz = sqrtf(__fmaf_rn(P[2], P[2], __fmaf_rn(P[1], P[1], 1.0f)));
+        const float wz = sqrt_n(__fmaf_rn(P[2], P[2], __fmaf_rn(P[1], P[1], 1.0f)));
 #pragma unroll
         for (int q = 0; q < 4; ++q) v[q] = (R)P[q];
-        v[4] = (R)(scalf / dV / wz);
+        v[4] = (R)(scalf * rcp_n(dV) * rcp_n(wz));
         return kind;
     }
 };
@@ -235,7 +235,7 @@ struct MixedC2p {
         const float im = 1.0f / mf;
         const float s1n = s1f * im, s2n = s2f * im, taun = tauf * im;
         const float ssn = s1n * s1n + s2n * s2n;
-        const float x1 = __fdividef(sqrtf(ssn), 1.0f + taun);   // |S| / (D + tau)
+        const float x1 = __fdividef(sqrt_n(ssn), 1.0f + taun);   // |S| / (D + tau)
         const bool valid = active && kind == HYDRO_NONE;
         const bool high = valid && x1 * x1 > high_thr;
         float guess = 0.0f;   // p / m
@@ -267,7 +267,7 @@ struct MixedC2p {
             // pass too, which keeps its FP64 primitive for the update's FP64
             // faces: this kernel stores no zone above the split. (Below 0.99 of
             // the split's W^2 the converged W cannot give such a velocity.)
-            const float inv_et = 1.0f / (taun + 1.0f + p32);
+            const float inv_et = rcp_n(taun + 1.0f + p32);
             fp64 = high_zone(w32 * s1n * inv_et, w32 * s2n * inv_et, a.uu_high_f);
         }
         if (DEFER) {
@@ -291,9 +291,9 @@ struct MixedC2p {
             ++st.zones;
             st.it32 += (unsigned)it32;
             if (!fp64) {
-                const float inv_dv = 1.0f / dV;
-                const float inv_et = 1.0f / (taun + 1.0f + p32);
-                P[0] = mf / w32 * inv_dv;
+                const float inv_dv = rcp_n(dV);
+                const float inv_et = rcp_n(taun + 1.0f + p32);
+                P[0] = mf * rcp_n(w32) * inv_dv;
                 P[1] = w32 * s1n * inv_et;
                 P[2] = w32 * s2n * inv_et;
                 P[3] = p32 * mf * inv_dv;
@@ -320,8 +320,8 @@ struct MixedC2p {
             // W = sqrt(1 + u^2) with explicit fused operations: the same
             // products appear in the time-step reduction below, and a kernel
             // with or without that reduction must round W alike
-            const float wz = sqrtf(__fmaf_rn(P[2], P[2], __fmaf_rn(P[1], P[1], 1.0f)));
-            const float v[NFIELD] = {P[0], P[1], P[2], P[3], scalf / dV / wz};
+            const float wz = sqrt_n(__fmaf_rn(P[2], P[2], __fmaf_rn(P[1], P[1], 1.0f)));
+            const float v[NFIELD] = {P[0], P[1], P[2], P[3], scalf * rcp_n(dV) * rcp_n(wz)};
             store_prim<float>(B, i, j, v);
             // above the split: its FP64 primitive for the update's FP64 faces
             // (the deferring form stores no such zone: it defers every zone

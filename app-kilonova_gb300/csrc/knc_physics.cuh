@@ -291,49 +291,31 @@ __device__ __forceinline__ void riemann(const PhysT<R>& ph, const R* pl, const R
 }
 
 // ---- FP32 relativistic forms for the mixed stage ------------------------------
-// The quantities of srhd_side<float> for a face normal fixed at compile time,
-// with the reciprocals shared: 1/W from one rsqrt (W = W^2 / W, v_n = u_n / W,
-// 1 - v^2 = 1/W^2), 1/rho and 1/h once each.
-template <int AXIS>
-__device__ __forceinline__ void srhd_side_f32(const PhysT<float>& ph, float rho, float ur, float uq, float pre,
-                                              float s, Side<float>& S) {
-    const float uu = ur * ur + uq * uq;
-    const float w2 = 1.0f + uu;
-    const float iw = rsqrtf(w2);
-    const float w = w2 * iw;
-    const float pr = pre * (1.0f / rho);     // p / rho
-    const float h = 1.0f + pr * ph.gh;
-    const float d = rho * w;
-    const float m = d * h;
-    const float un = AXIS == 0 ? ur : uq;
-    const float ut = AXIS == 0 ? uq : ur;
-    const float vn = un * iw;
-    S.U[0] = d;
-    S.U[1] = m * ur;
-    S.U[2] = m * uq;
-    const float cs2 = ph.gm * pr * (1.0f / h);
-    const float omv2 = iw * iw;
-    const float v2 = uu * omv2;
-    const float k = 1.0f - cs2;
-    const float a = vn * k;
-    // tau without cancellation: p (gh W^2 - 1) + D u^2 / (W + 1)
-    S.U[3] = pre * (ph.gh * w2 - 1.0f) + d * uu * (1.0f / (w + 1.0f));
-    const float b = sqrtf(cs2 * omv2 * (omv2 + ut * ut * omv2 * k));
-    S.F[0] = S.U[0] * vn;
-    S.F[1] = AXIS == 0 ? S.U[1] * vn + pre : S.U[1] * vn;
-    S.F[2] = AXIS == 1 ? S.U[2] * vn + pre : S.U[2] * vn;
-    S.F[3] = (S.U[3] + pre) * vn;
-    const float inv = 1.0f / (1.0f - v2 * cs2);
-    S.lm = (a - b) * inv;
-    S.lp = (a + b) * inv;
-    S.sU = s * w;
-    S.sF = s * un;
-    S.vn = vn;
-    S.pre = pre;
+// Reciprocals and roots of numbers that are never subnormal (Lorentz factors,
+// enthalpies, 1 - v^2 cs^2, wave-speed differences, volumes in the stage's
+// length unit): one hardware instruction, without the scaling that the plain
+// forms put around it for subnormal operands. On normal numbers they give the
+// bits of 1.0f / x, sqrtf(x) and rsqrtf(x) as this unit compiles them, and
+// a * rcp_n(b) those of a / b (checked over every mantissa).
+__device__ __forceinline__ float rcp_n(float x) {
+    float r;
+    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
+    return r;
+}
+__device__ __forceinline__ float sqrt_n(float x) {
+    float r;
+    asm("sqrt.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
+    return r;
+}
+__device__ __forceinline__ float rsqrt_n(float x) {
+    float r;
+    asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
+    return r;
 }
 
 // Both sides of a face at once, on Blackwell's paired FP32 units: every
-// product, sum and fused multiply-add of srhd_side_f32 runs on the (left,
+// product, sum and fused multiply-add of the side's quantities (srhd_side<float>'s
+// with the reciprocals shared) runs on the (left,
 // right) pair as one instruction (__fmul2_rn / __fadd2_rn / __ffma2_rn, each
 // lane rounded like its scalar form); reciprocals and square roots stay
 // per lane.
@@ -348,7 +330,7 @@ __device__ __forceinline__ void srhd_sides_f32x2(const PhysT<float>& ph, const f
     const float2 pre = pair(pl[3], pr[3]), s = pair(sl, sr);
     const float2 uu = __ffma2_rn(ur, ur, __fmul2_rn(uq, uq));
     const float2 w2 = __fadd2_rn(one, uu);
-    const float2 iw = pair(rsqrtf(w2.x), rsqrtf(w2.y));
+    const float2 iw = pair(rsqrt_n(w2.x), rsqrt_n(w2.y));   // 1 / W, shared below
     const float2 w = __fmul2_rn(w2, iw);
     const float2 prr = __fmul2_rn(pre, pair(1.0f / rho.x, 1.0f / rho.y));   // p / rho
     const float2 h = __ffma2_rn(prr, bcast(ph.gh), one);
@@ -358,18 +340,18 @@ __device__ __forceinline__ void srhd_sides_f32x2(const PhysT<float>& ph, const f
     const float2 ut = AXIS == 0 ? uq : ur;
     const float2 vn = __fmul2_rn(un, iw);
     const float2 U1 = __fmul2_rn(m, ur), U2 = __fmul2_rn(m, uq);
-    const float2 cs2 = __fmul2_rn(__fmul2_rn(bcast(ph.gm), prr), pair(1.0f / h.x, 1.0f / h.y));
+    const float2 cs2 = __fmul2_rn(__fmul2_rn(bcast(ph.gm), prr), pair(rcp_n(h.x), rcp_n(h.y)));
     const float2 omv2 = __fmul2_rn(iw, iw);                                  // 1 - v^2
     const float2 v2 = __fmul2_rn(uu, omv2);
     const float2 k = __ffma2_rn(cs2, mone, one);                            // 1 - cs^2
     const float2 a = __fmul2_rn(vn, k);
     const float2 wp1 = __fadd2_rn(w, one);
-    const float2 t = __fmul2_rn(__fmul2_rn(rho, uu), pair(1.0f / wp1.x, 1.0f / wp1.y));   // rho u^2 / (W + 1)
+    const float2 t = __fmul2_rn(__fmul2_rn(rho, uu), pair(rcp_n(wp1.x), rcp_n(wp1.y)));   // rho u^2 / (W + 1)
     // tau without cancellation: p (gh W^2 - 1) + W rho u^2 / (W + 1)
     const float2 U3 = __ffma2_rn(pre, __ffma2_rn(bcast(ph.gh), w2, mone), __fmul2_rn(w, t));
     const float2 inner = __ffma2_rn(__fmul2_rn(__fmul2_rn(ut, ut), omv2), k, omv2);
     const float2 barg = __fmul2_rn(__fmul2_rn(cs2, omv2), inner);
-    const float2 b = pair(sqrtf(barg.x), sqrtf(barg.y));
+    const float2 b = pair(sqrt_n(barg.x), sqrt_n(barg.y));
     // fluxes in the forms with the fewest roundings (all equal to U v_n + p e_n
     // in exact arithmetic): D v_n = rho u_n, S v_n = rho h u u_n,
     // (tau + p) v_n = u_n (rho u^2 / (W + 1) + gh p W); the density flux then
@@ -382,7 +364,7 @@ __device__ __forceinline__ void srhd_sides_f32x2(const PhysT<float>& ph, const f
     const float2 F2 = AXIS == 1 ? __ffma2_rn(rhohun, uq, pre) : __fmul2_rn(rhohun, uq);
     const float2 F3 = __fmul2_rn(un, __ffma2_rn(__fmul2_rn(bcast(ph.gh), pre), w, t));
     const float2 den = __ffma2_rn(__fmul2_rn(v2, cs2), mone, one);           // 1 - v^2 cs^2
-    const float2 inv = pair(1.0f / den.x, 1.0f / den.y);
+    const float2 inv = pair(rcp_n(den.x), rcp_n(den.y));
     const float2 lm = __fmul2_rn(__ffma2_rn(b, mone, a), inv);
     const float2 lp = __fmul2_rn(__fadd2_rn(a, b), inv);
     const float2 sU = __fmul2_rn(s, w), sF = __fmul2_rn(s, un);
@@ -415,7 +397,7 @@ __device__ __forceinline__ void hlle_f32x2(const Side<float>& L, const Side<floa
         for (int q = 0; q < 4; ++q) out[q] = R.F[q];
         out[4] = R.sF;
     } else {
-        const float inv = 1.0f / (ap - am);
+        const float inv = rcp_n(ap - am);
         const float apam = ap * am;
         const float2 AP = bcast(ap), MAM = bcast(-am), APAM = bcast(apam), INV = bcast(inv);
 #pragma unroll
@@ -445,7 +427,7 @@ __device__ __forceinline__ void sources_srhd_f32(const PhysT<float>& ph, const f
                                                  float S[4]) {
     const float rho = P[0], ur = P[1], uq = P[2], pre = P[3];
     const float mass = rho + pre * ph.gh;
-    const float ir = 1.0f / r;
+    const float ir = rcp_n(r);
     S[0] = 0.0f;
     S[1] = (2.0f * pre + mass * uq * uq) * ir;
     S[2] = (pre * cot - mass * ur * uq) * ir;
@@ -549,17 +531,22 @@ __device__ __forceinline__ bool newton_fast(R m, R ss, R tau, R gm, R p, R tol_a
     const R bmax = sizeof(R) == 8 ? R(1.0 - 1e-10) : R(1.0f - 1e-6f);
     for (int n = 0; n < maxit; ++n) {
         const R et = tau + p + m;
-        const R inv = R(1) / et;
+        R inv, w;
+        if constexpr (sizeof(R) == 4) inv = rcp_n(et);
+        else inv = R(1) / et;
         const R b2 = rmin(ss * inv * inv, bmax);
         const R omb = R(1) - b2;
-        const R w = sizeof(R) == 8 ? (R)rsqrt((double)omb) : (R)rsqrtf((float)omb);
+        if constexpr (sizeof(R) == 4) w = rsqrt_n(omb);
+        else w = rsqrt(omb);
         const R w2 = w * w;
         const R X = tau + m * (R(1) - w) + p * (R(1) - w2);
         const R de = X * omb;
         const R f = (gm - R(1)) * de - p;
         const R dh = m * omb * w + de + p;
         const R den = b2 * gm * p - dh;
-        const R step = f * dh / den;
+        R step;
+        if constexpr (sizeof(R) == 4) step = __fmul_rn(__fmul_rn(f, dh), rcp_n(den));
+        else step = f * dh / den;
         p = p - step;
         iters = n + 1;
         if (rabs(f) < tol_abs || rabs(step) <= tol_rel * rabs(p)) {
