@@ -76,16 +76,16 @@ struct Fp64Recovery {
     int it64;
     int fbs;
     int it32;
+    double root;   // the volume-integrated pressure, when the FP64 iteration found it (else 0)
 };
 
 __device__ __forceinline__ Fp64Recovery recover_fp64(const StageArgs& a, double m, double s1, double s2, double tau,
                                                      float dV, bool ok32, float p32) {
-    Fp64Recovery r = {{0.f, 0.f, 0.f, 0.f}, HYDRO_NONE, 0, 0, 0};
+    Fp64Recovery r = {{0.f, 0.f, 0.f, 0.f}, HYDRO_NONE, 0, 0, 0, 0.0};
     const double ss = s1 * s1 + s2 * s2;
     const double tol = NEWTON_TOLERANCE * (m + tau);
     double p64 = 0.0, w64 = 1.0;
-    const bool ok = newton_fast<double>(m, ss, tau, a.gm, ok32 ? (double)p32 * m : 0.0, tol, 0.0, NEWTON_ITER_MAX,
-                                        p64, w64, r.it64);
+    const bool ok = newton_fast64(m, ss, tau, a.gm, ok32 ? (double)p32 * m : 0.0, tol, p64, w64, r.it64);
     if (!ok) {
         // fallback: the reference's iteration from the plain guess
         r.fbs = 1;
@@ -99,16 +99,17 @@ __device__ __forceinline__ Fp64Recovery recover_fp64(const StageArgs& a, double 
             r.kind = kf;
         } else {
             // Pd is the (floored) primitive of the volume-integrated state
-            const double inv_dv = a.lscale3_d / (double)dV;
+            const double inv_dv = div64(a.lscale3_d, f2d(dV));
             r.P[0] = (float)(Pd[0] * inv_dv);
             r.P[1] = (float)Pd[1];
             r.P[2] = (float)Pd[2];
             r.P[3] = (float)(Pd[3] * inv_dv);
         }
     } else {
-        const double inv_dv = a.lscale3_d / (double)dV;
-        const double inv_et = 1.0 / (tau + m + p64);
-        const double rho = m / w64 * inv_dv;
+        const double inv_dv = div64(a.lscale3_d, f2d(dV));
+        const double inv_et = div64(1.0, tau + m + p64);
+        const double rho = div64(m, w64) * inv_dv;
+        r.root = p64;
         r.P[0] = (float)rho;
         r.P[1] = (float)(w64 * s1 * inv_et);
         r.P[2] = (float)(w64 * s2 * inv_et);
@@ -128,7 +129,7 @@ static __device__ __noinline__ Fp64Recovery recover_fp64_call(const StageArgs& a
     int it32 = 0;
     if (run32) {
         float w32 = 1.f;
-        ok32 = newton_fast<float>(1.0f, ssn, taun, a.gm_f, guess, 2e-7f * taun, 1e-6f, 16, p32, w32, it32);
+        ok32 = newton_fast(1.0f, ssn, taun, a.gm_f, guess, 2e-7f * taun, 1e-6f, 16, p32, w32, it32);
     }
     const int64_t n = (int64_t)B.nr * B.nq;
     const double* Ub = B.buf[a.sel_in] + (int64_t)i * B.nq + j;
@@ -159,7 +160,7 @@ struct MixedRemapRecovery {
         const bool high = x1 * x1 > a.high_thr_f;
         float p32 = 0.f, w32 = 1.f;
         int it32 = 0;
-        const bool ok32 = newton_fast<float>(1.0f, ssn, taun, a.gm_f, 0.0f, 2e-7f * taun, 1e-6f, 16, p32, w32, it32);
+        const bool ok32 = newton_fast(1.0f, ssn, taun, a.gm_f, 0.0f, 2e-7f * taun, 1e-6f, 16, p32, w32, it32);
         float P[4];
         int kind = HYDRO_NONE;
         if (!high && ok32) {
@@ -259,7 +260,7 @@ struct MixedC2p {
         // density L1 unchanged). The deferring form leaves the high zones'
         // iteration to the dense pass.
         if (valid && !(DEFER && high))
-            ok32 = newton_fast<float>(1.0f, ssn, taun, gmf, guess, 2e-7f * taun, 1e-6f, 16, p32, w32, it32);
+            ok32 = newton_fast(1.0f, ssn, taun, gmf, guess, 2e-7f * taun, 1e-6f, 16, p32, w32, it32);
         bool fp64 = valid && (high || !ok32);
         if (DEFER && valid && !fp64 && w32 * w32 > 0.99f * (a.uu_high_f + 1.0f)) {
             // a zone whose stored FP32 four-velocity would be above the split
@@ -287,6 +288,7 @@ struct MixedC2p {
             }
         }
         float P[4] = {0.f, 0.f, 0.f, 0.f};
+        double root = 0.0;   // an FP64 root of the pressure, if one was found
         if (valid) {
             ++st.zones;
             st.it32 += (unsigned)it32;
@@ -308,6 +310,7 @@ struct MixedC2p {
 #pragma unroll
                 for (int q = 0; q < 4; ++q) P[q] = r.P[q];
                 kind = r.kind;
+                root = r.root;
                 st.it64 += (unsigned)r.it64;
                 st.fbs += (unsigned)r.fbs;
             }
@@ -327,7 +330,7 @@ struct MixedC2p {
             // (the deferring form stores no such zone: it defers every zone
             // above the split, and its list holds every zone of the layout)
             if constexpr (!DEFER) {
-                if (high_zone(P[1], P[2], a.uu_high_f)) hp_store(a, slot, B, i, j, v);
+                if (high_zone(P[1], P[2], a.uu_high_f)) hp_store(a, slot, B, i, j, v, root);
             }
             if ((DT < 0 ? a.compute_dt != 0 : DT > 0) && kind == HYDRO_NONE) {
                 // State::time_step (src/state.rs:151-160) on this stage's

@@ -519,34 +519,27 @@ __device__ __forceinline__ int srhd_c2p_newton_plain(double gm, const double* U,
     return HYDRO_NONE;
 }
 
-// Newton-Raphson on the pressure, the reference's iteration rewritten with two
-// divisions: with X = tau + m (1 - W) + p (1 - W^2) and 1 - v^2 = 1/W^2,
+// Newton-Raphson on the pressure in FP32, the reference's iteration rewritten
+// with two divisions: with X = tau + m (1 - W) + p (1 - W^2) and 1 - v^2 = 1/W^2,
 // rho e = X / W^2, f = (gamma - 1) rho e - p, rho h = m / W + rho e + p and
 // f / f' = f rho h / (v^2 gamma p - rho h). Converged when |f| < tol_abs or the
-// step is below tol_rel |p| (FP32 only; tol_rel = 0 reproduces the reference's
-// criterion). Returns the root and W at the last evaluated pressure.
-template <class R>
-__device__ __forceinline__ bool newton_fast(R m, R ss, R tau, R gm, R p, R tol_abs, R tol_rel, int maxit, R& p_out,
-                                            R& w_out, int& iters) {
-    const R bmax = sizeof(R) == 8 ? R(1.0 - 1e-10) : R(1.0f - 1e-6f);
+// step is below tol_rel |p|. Returns the root and W at the last evaluated
+// pressure. (newton_fast64, knc_physics64.cuh, is its FP64 form.)
+__device__ __forceinline__ bool newton_fast(float m, float ss, float tau, float gm, float p, float tol_abs,
+                                            float tol_rel, int maxit, float& p_out, float& w_out, int& iters) {
     for (int n = 0; n < maxit; ++n) {
-        const R et = tau + p + m;
-        R inv, w;
-        if constexpr (sizeof(R) == 4) inv = rcp_n(et);
-        else inv = R(1) / et;
-        const R b2 = rmin(ss * inv * inv, bmax);
-        const R omb = R(1) - b2;
-        if constexpr (sizeof(R) == 4) w = rsqrt_n(omb);
-        else w = rsqrt(omb);
-        const R w2 = w * w;
-        const R X = tau + m * (R(1) - w) + p * (R(1) - w2);
-        const R de = X * omb;
-        const R f = (gm - R(1)) * de - p;
-        const R dh = m * omb * w + de + p;
-        const R den = b2 * gm * p - dh;
-        R step;
-        if constexpr (sizeof(R) == 4) step = __fmul_rn(__fmul_rn(f, dh), rcp_n(den));
-        else step = f * dh / den;
+        const float et = tau + p + m;
+        const float inv = rcp_n(et);
+        const float b2 = rmin(ss * inv * inv, 1.0f - 1e-6f);
+        const float omb = 1.0f - b2;
+        const float w = rsqrt_n(omb);
+        const float w2 = w * w;
+        const float X = tau + m * (1.0f - w) + p * (1.0f - w2);
+        const float de = X * omb;
+        const float f = (gm - 1.0f) * de - p;
+        const float dh = m * omb * w + de + p;
+        const float den = b2 * gm * p - dh;
+        const float step = __fmul_rn(__fmul_rn(f, dh), rcp_n(den));
         p = p - step;
         iters = n + 1;
         if (rabs(f) < tol_abs || rabs(step) <= tol_rel * rabs(p)) {

@@ -509,6 +509,47 @@ __device__ __forceinline__ double over_lorentz64(double x, double ur, double uq)
     return fp64_div(x, fp64_sqrt(w2, y), y);
 }
 
+// a / b
+static __device__ __noinline__ double div_plain(double a, double b) { return a / b; }
+__device__ __forceinline__ double div64(double a, double b) {
+    if (fp64_odd_numerator(a) || fp64_odd_divisor(b)) return div_plain(a, b);
+    return fp64_div(a, b, rcp_start(b));
+}
+
+// newton_fast in FP64 (the criterion on the residual alone) with its reciprocals, square root and
+// comparisons off the FP64 pipe; false also for operands outside the fast range
+// (the callers then take the plain recovery).
+__device__ __forceinline__ bool newton_fast64(double m, double ss, double tau, double gm, double p, double tol,
+                                              double& p_out, double& w_out, int& iters) {
+    const double bmax = 1.0 - 1e-10;
+    for (int n = 0; n < NEWTON_ITER_MAX; ++n) {
+        const double et = tau + p + m;
+        if (fp64_odd_divisor(et)) return false;
+        const double inv = fp64_rcp(et, rcp_start(et));
+        double b2 = ss * inv * inv;
+        if (magnitude(b2) >= (unsigned long long)__double_as_longlong(bmax)) b2 = bmax;
+        const double omb = 1.0 - b2;
+        const Start64 y = rsqrt_start(omb);
+        const double r = fp64_sqrt(omb, y);
+        const double w = fp64_rcp(r, y);
+        const double X = tau + m * (1.0 - w) + p * (1.0 - w * w);
+        const double de = X * omb;
+        const double f = (gm - 1.0) * de - p;
+        const double dh = m * omb * w + de + p;
+        const double den = b2 * gm * p - dh;
+        const double num = f * dh;
+        if (fp64_odd_divisor(den) || fp64_odd_numerator(num)) return false;
+        p = p - fp64_div(num, den, rcp_start(den));
+        iters = n + 1;
+        if (magnitude(f) < magnitude(tol)) {
+            p_out = p;
+            w_out = w;
+            return !is_nan_bits(p);
+        }
+    }
+    return false;
+}
+
 // Max signal speed of a primitive state (max_signal_speed).
 __device__ __forceinline__ double max_signal_speed64(const PhysT<double>& ph, const double* P) {
     bool odd = false;
