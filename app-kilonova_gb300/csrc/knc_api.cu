@@ -231,30 +231,37 @@ void free_block(BlockH& b) {
 // 1.358, 1.379 ms).
 constexpr int STREAM_STRIP_ROWS = 4;
 
-// Rows of an FP64 update item (32 columns each, knc_f64_update.cu) where the
-// caller has not chosen them. The update's time is the FP64 instructions of
-// the SM that gets the most CTAs (4 items each): an item costs about one row's
-// instructions before its march (the edges and the first face) and then one
-// per row, and a CTA alone on its SM runs a fifth slower (nothing hides its
-// other instructions). The rows that make that least.
-int64_t f64_update_rows(const std::vector<std::pair<int64_t, int64_t>>& shapes, int sms) {
-    int64_t best = 1;
-    double least = -1.0;
-    for (int64_t rows = 1; rows <= 32; ++rows) {
-        int64_t items = 0, most = 0;
-        for (const auto& s : shapes) {
-            const int64_t per = (s.first + rows - 1) / rows;
-            items += per * ((s.second + TILE_Q - 1) / TILE_Q);
-            most = std::max(most, (s.first + per - 1) / per);
-        }
-        const int64_t ctas = (items + 3) / 4, on_sm = (ctas + sms - 1) / sms;
-        const double cost = (double)on_sm * ((double)most + 1.1) * (on_sm == 1 ? 1.2 : 1.0);
-        if (least < 0.0 || cost < least) {
-            least = cost;
-            best = rows;
+// The FP64 update's items {slot, i0, j0, rows} (32 columns each,
+// knc_f64_update.cu) of the blocks slot0, slot0 + 1, ... with the given (nr,
+// nq), where the caller has not chosen their rows. An item costs about one
+// row's instructions before its march (its edges and first face), which asks
+// for many rows; the SMs take CTAs of 4 items in list order, and the last ones
+// run on a machine that empties, which asks for few. So the rows follow the
+// work left (guided self-scheduling, Polychronopoulos and Kuck 1987): the rows
+// left per SM partition over 1.5, at most 16, at least 2. 2048 x 512 jet fold
+// 5.22 (8 rows throughout) -> 4.78 ms, over 1, 2, 3: 4.74, 4.94, 5.00;
+// Newtonian sphere 4.12 -> 3.83 ms. Grids under 16 rows per partition take 2
+// throughout (450 x 230, RK3: 2 rows 1.10 ms, 3 to 4 1.18, 1 1.36; 256 x 128:
+// 2 rows 235 us, 1 229, 3 267).
+constexpr double F64_ROWS_OVER = 1.5, F64_ROWS_LEAST = 2.0, F64_ROWS_MOST = 16.0, F64_ROWS_SMALL_GRID = 16.0;
+
+std::vector<int4> f64_items(const std::vector<std::pair<int64_t, int64_t>>& shapes, int slot0, int sms) {
+    double left = 0.0;   // rows of 32 columns left, per SM partition
+    for (const auto& s : shapes) left += (double)(s.first * ((s.second + TILE_Q - 1) / TILE_Q)) / (4.0 * sms);
+    const double most = left < F64_ROWS_SMALL_GRID ? F64_ROWS_LEAST : F64_ROWS_MOST;
+    std::vector<int4> items;
+    for (size_t k = 0; k < shapes.size(); ++k) {
+        const int64_t nr = shapes[k].first, nq = shapes[k].second, cols = (nq + TILE_Q - 1) / TILE_Q;
+        for (int64_t i0 = 0; i0 < nr;) {
+            const int64_t want = (int64_t)std::min(std::max(left / F64_ROWS_OVER, F64_ROWS_LEAST), most);
+            const int64_t per = (nr - i0 + want - 1) / want, rows = (nr - i0 + per - 1) / per;
+            for (int64_t j0 = 0; j0 < nq; j0 += TILE_Q)
+                items.push_back(make_int4(slot0 + (int)k, (int)i0, (int)j0, (int)rows));
+            i0 += rows;
+            left -= (double)(rows * cols) / (4.0 * sms);
         }
     }
-    return best;
+    return items;
 }
 
 // One block set's device view.
@@ -270,7 +277,7 @@ struct Layout {
     int utr = 0;
     int uform = -1;
     int list_cols = 0;          // columns of a strip: 32 for the FP64 update's items, else STRIP_OUT
-    bool list_auto = false;     // item rows by f64_update_rows
+    bool list_auto = false;     // item rows by f64_items
     int64_t nzones = 0;         // zones of the block set
     TmaMaps* d_tmaps = nullptr; // tensor maps per slot (tiles of `utr` rows), when every block allows them
     int tmaps_cap = 0;
@@ -666,11 +673,7 @@ int rebuild_table(knc_ctx* c) {
     if (!c->dirty && L(c).utr == c->utr && L(c).uform == c->uform && L(c).chunk_nt == fused_threads(c) &&
         L(c).list_cols == cols && L(c).list_auto == rows_auto)
         return KNC_OK;
-    std::vector<std::pair<int64_t, int64_t>> shapes;
-    for (auto& kv : c->blocks) shapes.push_back({kv.second.nr, kv.second.nq});
-    const int64_t auto_rows = rows64 ? f64_update_rows(shapes, c->sms) : 0;
-    const int64_t item_rows = rows_auto ? auto_rows : rows64 ? std::min<int64_t>(c->utr, 32) : c->utr;
-    const int64_t stream_rows = rows64 ? auto_rows : STREAM_STRIP_ROWS;
+    const int64_t item_rows = rows64 ? std::min<int64_t>(c->utr, 32) : c->utr;
     L(c).list_cols = cols;
     L(c).list_auto = rows_auto;
     const int nb = (int)c->blocks.size();
@@ -745,11 +748,10 @@ int rebuild_table(knc_ctx* c) {
         L(c).strip_off.push_back((int)strips.size());
         L(c).sstrip_off.push_back((int)sstrips.size());
         L(c).zone_off.push_back(zoff);
-        // (FP64: as even as whole rows allow)
-        const int64_t sper = (b.nr + stream_rows - 1) / stream_rows, sh = rows64 ? (b.nr + sper - 1) / sper : stream_rows;
-        for (int64_t j0 = 0; j0 < b.nq; j0 += cols)
-            for (int64_t i0 = 0; i0 < b.nr; i0 += sh)
-                sstrips.push_back(make_int4(slot, (int)i0, (int)j0, (int)std::min<int64_t>(sh, b.nr - i0)));
+        for (int64_t j0 = 0; j0 < b.nq && !rows64; j0 += STRIP_OUT)
+            for (int64_t i0 = 0; i0 < b.nr; i0 += STREAM_STRIP_ROWS)
+                sstrips.push_back(
+                    make_int4(slot, (int)i0, (int)j0, (int)std::min<int64_t>(STREAM_STRIP_ROWS, b.nr - i0)));
         for (int64_t i0 = 0; i0 < b.nr; i0 += TILE_R)
             for (int64_t j0 = 0; j0 < b.nq; j0 += TILE_Q)
                 tiles.push_back(make_int4(slot, (int)i0, (int)j0, (int)zoff));
@@ -763,12 +765,10 @@ int rebuild_table(knc_ctx* c) {
                     strips.push_back(make_int4(slot, (int)i0, (int)j0, (int)rows));
                     i0 += rows;
                 }
-        } else {
-            const int64_t per = (b.nr + item_rows - 1) / item_rows;
-            const int64_t th = rows_auto ? (b.nr + per - 1) / per : item_rows;
-            for (int64_t i0 = 0; i0 < b.nr; i0 += th)
+        } else if (!rows_auto) {
+            for (int64_t i0 = 0; i0 < b.nr; i0 += item_rows)
                 for (int64_t j0 = 0; j0 < b.nq; j0 += TILE_Q)
-                    utiles.push_back(make_int4(slot, (int)i0, (int)j0, (int)std::min<int64_t>(th, b.nr - i0)));
+                    utiles.push_back(make_int4(slot, (int)i0, (int)j0, (int)std::min<int64_t>(item_rows, b.nr - i0)));
         }
         if (tma_ok) tma_ok = c->utr <= 16 && encode_block_maps(b, c->utr, &maps[k]);
         for (int64_t z0 = 0; z0 < b.nr * b.nq; z0 += nt)
@@ -777,6 +777,11 @@ int rebuild_table(knc_ctx* c) {
         zoff += b.nr * b.nq;
         prev = &b;
         ++slot;
+    }
+    if (rows_auto) {
+        std::vector<std::pair<int64_t, int64_t>> shapes;
+        for (const BlockH* b : order) shapes.push_back({b->nr, b->nq});
+        utiles = f64_items(shapes, 0, c->sms);
     }
     L(c).tile_off.push_back((int)tiles.size());
     L(c).utile_off.push_back((int)utiles.size());
@@ -2359,8 +2364,15 @@ int build_chunks(knc_ctx* c, int S) {
     for (int k = 0; k < G; ++k)
         for (int s = 0; s < S; ++s) {
             l.sc_strip_off.push_back((int)strips.size());
-            strips.insert(strips.end(), l.sstrips_h.begin() + l.sstrip_off[cb[k]],
-                          l.sstrips_h.begin() + l.sstrip_off[cb[k + 1]]);
+            if (l.list_cols == TILE_Q) {   // the FP64 update's items
+                std::vector<std::pair<int64_t, int64_t>> shapes;
+                for (int b = cb[k]; b < cb[k + 1]; ++b) shapes.push_back({l.tab_h[b].nr, l.tab_h[b].nq});
+                const std::vector<int4> items = f64_items(shapes, cb[k], c->sms);
+                strips.insert(strips.end(), items.begin(), items.end());
+            } else {
+                strips.insert(strips.end(), l.sstrips_h.begin() + l.sstrip_off[cb[k]],
+                              l.sstrips_h.begin() + l.sstrip_off[cb[k + 1]]);
+            }
             const int rows = 2 * S - 2 * s - 2;
             if (rows <= 0) continue;
             for (int n : of_chunk[k]) {
