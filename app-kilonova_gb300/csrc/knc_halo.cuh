@@ -117,13 +117,11 @@ static __device__ __noinline__ void ghost_zone(const GhostArgs& a, int end, int 
 // ---- FP64 primitives of the mixed stage's zones above the Lorentz-factor split
 // FP64 primitive (rho, u_r, u_theta, p, s) of the volume integrals U over the
 // FP64 volume dv: Newton on the pressure to the reference's residual
-// |f| < 1e-12 (D + tau) from `root`, the recovery's FP64 root of the same
-// volume integrals, or where it has none (0) from the stored FP32 pressure
-// pf[3] (a start one or two iterations from the root); the reference's
-// iteration from the plain guess as the fallback, the stored FP32 primitive if
-// both fail.
+// |f| < 1e-12 (D + tau) from the stored FP32 pressure pf[3] (a start one or
+// two iterations from the root), the reference's iteration from the plain
+// guess as the fallback, the stored FP32 primitive if both fail.
 __device__ __forceinline__ void recover_hp(const double gm, const double (&U)[5], double dv, const float (&pf)[NFIELD],
-                                           double root, double (&v)[NFIELD]) {
+                                           double (&v)[NFIELD]) {
 #pragma unroll
     for (int q = 0; q < NFIELD; ++q) v[q] = (double)pf[q];
     const double m = U[0], s1 = U[1], s2 = U[2], tau = U[3];
@@ -131,8 +129,7 @@ __device__ __forceinline__ void recover_hp(const double gm, const double (&U)[5]
     const double ss = s1 * s1 + s2 * s2;
     double p = 0.0, w = 1.0;
     int it = 0;
-    if (newton_fast64(m, ss, tau, gm, root != 0.0 ? root : (double)pf[3] * dv, NEWTON_TOLERANCE * (m + tau), p, w,
-                      it)) {
+    if (newton_fast64(m, ss, tau, gm, (double)pf[3] * dv, NEWTON_TOLERANCE * (m + tau), p, w, it)) {
         const double inv_et = div64(1.0, tau + m + p);
         v[0] = div64(div64(m, w), dv);
         v[1] = w * s1 * inv_et;
@@ -163,12 +160,12 @@ __device__ __forceinline__ void store_row_zone(T* P, int nr, int nq, int prow, i
 // view store_prim wrote it to (its own rows and the neighbours' halo rows),
 // each listed for the update's FP64 faces.
 __device__ __forceinline__ void hp_store(const StageArgs& a, int slot, const DevBlock& B, int i, int j,
-                                         const float (&pf)[NFIELD], double root) {
+                                         const float (&pf)[NFIELD]) {
     const int64_t n = (int64_t)B.nr * B.nq, z = (int64_t)i * B.nq + j;
     const double* Ub = B.buf[a.sel_in] + z;
     const double U[5] = {Ub[0], Ub[n], Ub[2 * n], Ub[3 * n], Ub[4 * n]};
     double v[NFIELD];
-    recover_hp(a.gm, U, B.dv[z], pf, root, v);
+    recover_hp(a.gm, U, B.dv[z], pf, v);
     store_row_zone(B.P64, B.nr, B.nq, i + 2, j, v);
     if (a.hp_list) note_high(a.hp_list, a.hp_count, a.hp_cap, slot, i + 2, B.nq, j);
     if (i < 2 && B.P_in_nbr) {
@@ -263,7 +260,7 @@ static __device__ __noinline__ void remap_zone(const StageArgs& a, const int4 it
                 float pf[NFIELD];
 #pragma unroll
                 for (int q = 0; q < NFIELD; ++q) pf[q] = (float)v[q];
-                recover_hp(a.gm, U, dv, pf, 0.0, v64);
+                recover_hp(a.gm, U, dv, pf, v64);
             }
             store_row_zone(T.P64, T.nr, nq_t, trow, j, v64);
             if (a.hp_list) note_high(a.hp_list, a.hp_count, a.hp_cap, it.x, trow, nq_t, j);

@@ -76,12 +76,11 @@ struct Fp64Recovery {
     int it64;
     int fbs;
     int it32;
-    double root;   // the volume-integrated pressure, when the FP64 iteration found it (else 0)
 };
 
 __device__ __forceinline__ Fp64Recovery recover_fp64(const StageArgs& a, double m, double s1, double s2, double tau,
                                                      float dV, bool ok32, float p32) {
-    Fp64Recovery r = {{0.f, 0.f, 0.f, 0.f}, HYDRO_NONE, 0, 0, 0, 0.0};
+    Fp64Recovery r = {{0.f, 0.f, 0.f, 0.f}, HYDRO_NONE, 0, 0, 0};
     const double ss = s1 * s1 + s2 * s2;
     const double tol = NEWTON_TOLERANCE * (m + tau);
     double p64 = 0.0, w64 = 1.0;
@@ -109,7 +108,6 @@ __device__ __forceinline__ Fp64Recovery recover_fp64(const StageArgs& a, double 
         const double inv_dv = div64(a.lscale3_d, f2d(dV));
         const double inv_et = div64(1.0, tau + m + p64);
         const double rho = div64(m, w64) * inv_dv;
-        r.root = p64;
         r.P[0] = (float)rho;
         r.P[1] = (float)(w64 * s1 * inv_et);
         r.P[2] = (float)(w64 * s2 * inv_et);
@@ -288,7 +286,6 @@ struct MixedC2p {
             }
         }
         float P[4] = {0.f, 0.f, 0.f, 0.f};
-        double root = 0.0;   // an FP64 root of the pressure, if one was found
         if (valid) {
             ++st.zones;
             st.it32 += (unsigned)it32;
@@ -310,7 +307,6 @@ struct MixedC2p {
 #pragma unroll
                 for (int q = 0; q < 4; ++q) P[q] = r.P[q];
                 kind = r.kind;
-                root = r.root;
                 st.it64 += (unsigned)r.it64;
                 st.fbs += (unsigned)r.fbs;
             }
@@ -330,7 +326,7 @@ struct MixedC2p {
             // (the deferring form stores no such zone: it defers every zone
             // above the split, and its list holds every zone of the layout)
             if constexpr (!DEFER) {
-                if (high_zone(P[1], P[2], a.uu_high_f)) hp_store(a, slot, B, i, j, v, root);
+                if (high_zone(P[1], P[2], a.uu_high_f)) hp_store(a, slot, B, i, j, v);
             }
             if ((DT < 0 ? a.compute_dt != 0 : DT > 0) && kind == HYDRO_NONE) {
                 // State::time_step (src/state.rs:151-160) on this stage's
