@@ -11,7 +11,7 @@
 // activations to bf16 as inference does, and the back-propagation is FP32
 // (straight-through for those roundings), with its three dense contractions on
 // the fifth-generation tensor cores (tcgen05.mma, accumulators in tensor
-// memory). Adam then updates the FP32 master weights.
+// memory). The launch's last CTA updates the FP32 master weights (Adam).
 #include <cuda_bf16.h>
 
 #include <algorithm>
@@ -28,10 +28,18 @@
 
 namespace knc {
 
-// ---- training kernel: one CTA of 128 threads per SM, a tile of 128 batch
-// rows at a time, thread t owning row t. The three 128 x 64 x K contractions
-// run on the tensor cores (tcgen05.mma, bf16 operands in shared memory, FP32
-// accumulators in tensor memory):
+// ---- training kernel: one CTA of 512 threads per SM, a tile of 128 batch
+// rows at a time; warp w holds rows 32 (w % 4) .. + 31 (the tensor memory lanes
+// it can read) and units 16 (w / 4) .. + 15 of each layer. Bound by instruction
+// fetch and latency: the per-row loops are unrolled (their values live in
+// registers), and with all 64 units of a row on one thread a launch ran
+// through 10000 instructions once, one warp per SM partition. A quarter of the
+// units per thread is a quarter of the code, run by four warps per partition,
+// and the last CTA takes the Adam step (200 steps of batch 8192 with 200000
+// pairs brought in: 7.7 ms, before 10.2 ms with Adam in a launch of its own; a
+// launch from a cold instruction cache 36 us, before 63). The three
+// 128 x 64 x K contractions run on the tensor cores (tcgen05.mma, bf16
+// operands in shared memory, FP32 accumulators in tensor memory):
 //   Z2  = A1 . W2^T                    (K = 64 hidden units)
 //   dA1 = dZ2 . W2                     (K = 64)
 //   dW2 += [dZ2_hi; dZ2_lo]^T . A1     (K = 128 rows, accumulated over tiles)
@@ -40,7 +48,9 @@ namespace knc {
 // lo = bf16(dZ2 - hi), which carries 16 of its 24 significand bits. The
 // per-unit sums (b1, W1, b2, W3, b3) are warp-shuffle reductions in FP32.
 constexpr int TC_ROWS = 128;                       // batch rows per tile = MMA M
-constexpr int TC_THREADS = 128;
+constexpr int TC_GROUPS = 4;                       // threads of a row, each with a quarter of the units
+constexpr int TC_UNITS = 64 / TC_GROUPS;
+constexpr int TC_THREADS = TC_ROWS * TC_GROUPS;
 constexpr uint32_t TC_TMEM_COLS = 256;             // Z2 at 0, dA1 at 64, dW2 at 128
 constexpr uint32_t TC_KLBO = 128, TC_KSBO = 1024;  // [rows][64] tiles: 8 K-chunks of 128 B per 8-row group
 constexpr uint32_t TC_TLBO = 144, TC_TSBO = 16 * 144;   // [n][128 rows] tiles: K-chunks 144 B apart
@@ -56,8 +66,17 @@ struct TcTrainSmem {
     unsigned char dzt[16 * TC_TSBO];          // [dZ2 hi; dZ2 lo]^T (M = 128: u, then 64 + u; K = row)
     float w1[MLP_H * 3], b1[MLP_H], b2[MLP_H], w3[MLP_H];
     float b3, xm[3], xs[3];
+    float part[TC_GROUPS][TC_ROWS];           // the groups' shares of a row's output
     uint64_t bar[2];
     uint32_t tmem_slot;
+    uint32_t last;                            // this CTA finished last (it takes the Adam step)
+};
+
+// Adam's state and this step's constants; w null: no step.
+struct AdamArgs {
+    float *w, *m, *v;
+    unsigned* done;     // CTAs that have added their gradients
+    float lr, b1, b2, eps, c1, c2;
 };
 
 // Byte offsets in the two operand layouts.
@@ -76,12 +95,13 @@ __device__ __forceinline__ void st_bf16(unsigned char* base, uint32_t off, __nv_
     *reinterpret_cast<__nv_bfloat16*>(base + off) = v;
 }
 
-// Sum over the warp's 32 rows of 32 per-row values: a butterfly that halves
-// the set at each of 5 exchanges; lane l ends with the sum of column l.
-__device__ __forceinline__ float warp_colsum32(float (&v)[32]) {
+// Sum over the warp's 32 rows of 16 per-row values: a butterfly that halves
+// the set at each of 4 exchanges, then one between lane pairs; lanes 2 c and
+// 2 c + 1 end with the sum of column c.
+__device__ __forceinline__ float warp_colsum16(float (&v)[TC_UNITS]) {
     const int lane = threadIdx.x & 31;
 #pragma unroll
-    for (int m = 16, h = 16; m > 0; m >>= 1, h >>= 1) {
+    for (int m = 16, h = 8; h > 0; m >>= 1, h >>= 1) {
         const bool up = (lane & m) != 0;
 #pragma unroll
         for (int k = 0; k < h; ++k) {
@@ -90,24 +110,27 @@ __device__ __forceinline__ float warp_colsum32(float (&v)[32]) {
             v[k] = keep + __shfl_xor_sync(0xffffffffu, send, m);
         }
     }
-    return v[0];
+    return v[0] + __shfl_xor_sync(0xffffffffu, v[0], 1);
 }
 
 // One launch = one gradient evaluation over `rows` rows. Row r reads data row
 // (seed ? hash(seed, r) % n_data : r). Gradients (of the mean loss) are added
 // into grad[]; the summed squared error into *loss_sum. A tensor-core wait
 // that gives up sets *err.
-__global__ void __launch_bounds__(TC_THREADS, 1) mlp_train_tc_kernel(const float* __restrict__ w,
+__global__ void __launch_bounds__(TC_THREADS, 1) mlp_train_tc_kernel(const float* w,
                                                                     const float* __restrict__ x,
                                                                     const float* __restrict__ y, int64_t n_data,
                                                                     int64_t rows, uint64_t seed, float inv_batch,
                                                                     float* __restrict__ grad,
                                                                     float* __restrict__ loss_sum,
-                                                                    float* __restrict__ pred, unsigned* err) {
+                                                                    float* __restrict__ pred, unsigned* err,
+                                                                    AdamArgs adam) {
     extern __shared__ unsigned char smem_raw[];
     TcTrainSmem& S =
         *reinterpret_cast<TcTrainSmem*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int rt = (warp & 3) * 32 + lane;      // this thread's row of the tile
+    const int grp = warp >> 2, u0 = grp * TC_UNITS;   // its units u0 .. u0 + 15
 
     for (int k = tid; k < MLP_H * MLP_H; k += TC_THREADS) {
         const int u = k >> 6, v = k & 63;
@@ -141,16 +164,15 @@ __global__ void __launch_bounds__(TC_THREADS, 1) mlp_train_tc_kernel(const float
     const uint32_t dzk0 = smem_u32(S.dzk[0]), dzk1 = smem_u32(S.dzk[1]);
     const uint32_t a1t = smem_u32(S.a1t), dzt = smem_u32(S.dzt);
 
-    // lane sums of columns lane and 32 + lane: W3, b2, b1, W1 (3)
-    float g_w3[2] = {0.f, 0.f}, g_b2[2] = {0.f, 0.f}, g_b1[2] = {0.f, 0.f};
-    float g_w1[3][2] = {{0.f, 0.f}, {0.f, 0.f}, {0.f, 0.f}};
+    // lane sums of column u0 + lane / 2: W3, b2, b1, W1 (3)
+    float g_w3 = 0.f, g_b2 = 0.f, g_b1 = 0.f, g_w1[3] = {0.f, 0.f, 0.f};
     float g_b3 = 0.f, l_sum = 0.f;
     uint32_t phase = 0;
     bool any_tile = false, failed = false;
 
     const int64_t ntiles = (rows + TC_ROWS - 1) / TC_ROWS;
     for (int64_t t = blockIdx.x; t < ntiles; t += gridDim.x) {
-        const int64_t r = t * TC_ROWS + tid;
+        const int64_t r = t * TC_ROWS + rt;
         const bool valid = r < rows;
         int64_t d = r;
         if (seed) d = (int64_t)(splitmix64(seed ^ splitmix64((uint64_t)r)) % (uint64_t)n_data);
@@ -169,22 +191,22 @@ __global__ void __launch_bounds__(TC_THREADS, 1) mlp_train_tc_kernel(const float
         };
         // ---- layer 1: A1 row (K-major) and column (transposed tile)
 #pragma unroll
-        for (int c = 0; c < 8; ++c) {
+        for (int c = 0; c < TC_UNITS / 8; ++c) {
             uint32_t pk[4];
 #pragma unroll
             for (int h = 0; h < 4; ++h) {
-                const int v = 8 * c + 2 * h;
+                const int v = u0 + 8 * c + 2 * h;
                 const float za = z1_of(v), zb = z1_of(v + 1);
                 const __nv_bfloat16 ba = __float2bfloat16_rn(za / (1.0f + expf(-za)));
                 const __nv_bfloat16 bb = __float2bfloat16_rn(zb / (1.0f + expf(-zb)));
-                st_bf16(S.a1t, tbyte(v, tid), ba);
-                st_bf16(S.a1t, tbyte(v + 1, tid), bb);
+                st_bf16(S.a1t, tbyte(v, rt), ba);
+                st_bf16(S.a1t, tbyte(v + 1, rt), bb);
                 __nv_bfloat162 p2;
                 p2.x = ba;
                 p2.y = bb;
                 pk[h] = *reinterpret_cast<const uint32_t*>(&p2);
             }
-            *reinterpret_cast<uint4*>(S.a1k + kbyte(tid, 8 * c)) = make_uint4(pk[0], pk[1], pk[2], pk[3]);
+            *reinterpret_cast<uint4*>(S.a1k + kbyte(rt, u0 + 8 * c)) = make_uint4(pk[0], pk[1], pk[2], pk[3]);
         }
         fence_proxy_async();
         tc_fence_before();
@@ -202,56 +224,62 @@ __global__ void __launch_bounds__(TC_THREADS, 1) mlp_train_tc_kernel(const float
             break;
         }
         tc_fence_after();
-        // ---- layer 2 and the output
-        float z2[64], s2[64];
-        tc_ld64(tmem, 0, z2);
+        // ---- layer 2 and the output (each group's units, then their sum)
+        float z2[TC_UNITS], s2[TC_UNITS];
+        tc_ld16(tmem + ((uint32_t)(warp & 3) << 21) + (uint32_t)u0, z2);
+        tc_wait_ld();
+        float share = 0.f;
+#pragma unroll
+        for (int u = 0; u < TC_UNITS; ++u) {
+            z2[u] += S.b2[u0 + u];
+            s2[u] = sigm(z2[u]);
+            share = fmaf(z2[u] * s2[u], S.w3[u0 + u], share);
+        }
+        S.part[grp][rt] = share;
+        __syncthreads();
         float out = S.b3;
 #pragma unroll
-        for (int u = 0; u < 64; ++u) {
-            z2[u] += S.b2[u];
-            s2[u] = sigm(z2[u]);
-            out = fmaf(z2[u] * s2[u], S.w3[u], out);
-        }
-        if (pred && valid && !seed) pred[r] = out;
+        for (int g = 0; g < TC_GROUPS; ++g) out += S.part[g][rt];
+        if (pred && valid && !seed && grp == 0) pred[r] = out;
         const float e = valid ? out - yr : 0.f;
-        l_sum += e * e;
         const float dout = 2.0f * e * inv_batch;
-        g_b3 += dout;
+        if (grp == 0) {
+            l_sum += e * e;
+            g_b3 += dout;
+        }
         // W3: dout h2 summed over rows
+        {
+            float q[TC_UNITS];
 #pragma unroll
-        for (int hh = 0; hh < 2; ++hh) {
-            float q[32];
-#pragma unroll
-            for (int k = 0; k < 32; ++k) q[k] = dout * (z2[32 * hh + k] * s2[32 * hh + k]);
-            g_w3[hh] += warp_colsum32(q);
+            for (int k = 0; k < TC_UNITS; ++k) q[k] = dout * (z2[k] * s2[k]);
+            g_w3 += warp_colsum16(q);
         }
         // dZ2 in place of z2
 #pragma unroll
-        for (int u = 0; u < 64; ++u) {
+        for (int u = 0; u < TC_UNITS; ++u) {
             const float s = s2[u];
-            z2[u] = dout * S.w3[u] * s * (1.0f + z2[u] * (1.0f - s));
+            z2[u] = dout * S.w3[u0 + u] * s * (1.0f + z2[u] * (1.0f - s));
         }
+        {
+            float q[TC_UNITS];
 #pragma unroll
-        for (int hh = 0; hh < 2; ++hh) {
-            float q[32];
-#pragma unroll
-            for (int k = 0; k < 32; ++k) q[k] = z2[32 * hh + k];
-            g_b2[hh] += warp_colsum32(q);
+            for (int k = 0; k < TC_UNITS; ++k) q[k] = z2[k];
+            g_b2 += warp_colsum16(q);
         }
         // dZ2 = hi + lo into the row tiles (dA1) and the stacked transposed tile (dW2)
 #pragma unroll
-        for (int c = 0; c < 8; ++c) {
+        for (int c = 0; c < TC_UNITS / 8; ++c) {
             uint32_t ph[4], pl[4];
 #pragma unroll
             for (int h = 0; h < 4; ++h) {
-                const int u = 8 * c + 2 * h;
-                const __nv_bfloat16 ha = __float2bfloat16_rn(z2[u]), hb = __float2bfloat16_rn(z2[u + 1]);
-                const __nv_bfloat16 la = __float2bfloat16_rn(z2[u] - __bfloat162float(ha));
-                const __nv_bfloat16 lb = __float2bfloat16_rn(z2[u + 1] - __bfloat162float(hb));
-                st_bf16(S.dzt, tbyte(u, tid), ha);
-                st_bf16(S.dzt, tbyte(u + 1, tid), hb);
-                st_bf16(S.dzt, tbyte(64 + u, tid), la);
-                st_bf16(S.dzt, tbyte(64 + u + 1, tid), lb);
+                const int k = 8 * c + 2 * h, u = u0 + k;
+                const __nv_bfloat16 ha = __float2bfloat16_rn(z2[k]), hb = __float2bfloat16_rn(z2[k + 1]);
+                const __nv_bfloat16 la = __float2bfloat16_rn(z2[k] - __bfloat162float(ha));
+                const __nv_bfloat16 lb = __float2bfloat16_rn(z2[k + 1] - __bfloat162float(hb));
+                st_bf16(S.dzt, tbyte(u, rt), ha);
+                st_bf16(S.dzt, tbyte(u + 1, rt), hb);
+                st_bf16(S.dzt, tbyte(64 + u, rt), la);
+                st_bf16(S.dzt, tbyte(64 + u + 1, rt), lb);
                 __nv_bfloat162 p2;
                 p2.x = ha;
                 p2.y = hb;
@@ -260,8 +288,8 @@ __global__ void __launch_bounds__(TC_THREADS, 1) mlp_train_tc_kernel(const float
                 p2.y = lb;
                 pl[h] = *reinterpret_cast<const uint32_t*>(&p2);
             }
-            *reinterpret_cast<uint4*>(S.dzk[0] + kbyte(tid, 8 * c)) = make_uint4(ph[0], ph[1], ph[2], ph[3]);
-            *reinterpret_cast<uint4*>(S.dzk[1] + kbyte(tid, 8 * c)) = make_uint4(pl[0], pl[1], pl[2], pl[3]);
+            *reinterpret_cast<uint4*>(S.dzk[0] + kbyte(rt, u0 + 8 * c)) = make_uint4(ph[0], ph[1], ph[2], ph[3]);
+            *reinterpret_cast<uint4*>(S.dzk[1] + kbyte(rt, u0 + 8 * c)) = make_uint4(pl[0], pl[1], pl[2], pl[3]);
         }
         fence_proxy_async();
         tc_fence_before();
@@ -283,6 +311,14 @@ __global__ void __launch_bounds__(TC_THREADS, 1) mlp_train_tc_kernel(const float
             tc_commit(smem_u32(&S.bar[1]));
         }
         any_tile = true;
+        // silu'(z1) of the backward pass, while the tensor core works
+        float ds[TC_UNITS];
+#pragma unroll
+        for (int v = 0; v < TC_UNITS; ++v) {
+            const float z = z1_of(u0 + v);
+            const float s = sigm(z);
+            ds[v] = s * (1.0f + z * (1.0f - s));
+        }
         if (__syncthreads_or(!mbar_wait_bounded(&S.bar[1], phase, TC_WAIT_POLLS))) {
             failed = true;
             break;
@@ -290,30 +326,23 @@ __global__ void __launch_bounds__(TC_THREADS, 1) mlp_train_tc_kernel(const float
         tc_fence_after();
         phase ^= 1u;
         // ---- layer 1 backward: dz1 = dA1 silu'(z1), in place of dA1
-        float da[64];
-        tc_ld64(tmem, 64, da);
+        float da[TC_UNITS], q[TC_UNITS];
+        tc_ld16(tmem + ((uint32_t)(warp & 3) << 21) + 64u + (uint32_t)u0, da);
+        tc_wait_ld();
 #pragma unroll
-        for (int v = 0; v < 64; ++v) {
-            const float z = z1_of(v);
-            const float s = sigm(z);
-            da[v] = da[v] * s * (1.0f + z * (1.0f - s));
-        }
+        for (int v = 0; v < TC_UNITS; ++v) da[v] *= ds[v];
 #pragma unroll
-        for (int hh = 0; hh < 2; ++hh) {
-            float q[32];
+        for (int k = 0; k < TC_UNITS; ++k) q[k] = da[k];
+        g_b1 += warp_colsum16(q);
 #pragma unroll
-            for (int k = 0; k < 32; ++k) q[k] = da[32 * hh + k];
-            g_b1[hh] += warp_colsum32(q);
+        for (int k = 0; k < TC_UNITS; ++k) q[k] = da[k] * xn0;
+        g_w1[0] += warp_colsum16(q);
 #pragma unroll
-            for (int k = 0; k < 32; ++k) q[k] = da[32 * hh + k] * xn0;
-            g_w1[0][hh] += warp_colsum32(q);
+        for (int k = 0; k < TC_UNITS; ++k) q[k] = da[k] * xn1;
+        g_w1[1] += warp_colsum16(q);
 #pragma unroll
-            for (int k = 0; k < 32; ++k) q[k] = da[32 * hh + k] * xn1;
-            g_w1[1][hh] += warp_colsum32(q);
-#pragma unroll
-            for (int k = 0; k < 32; ++k) q[k] = da[32 * hh + k] * xn2;
-            g_w1[2][hh] += warp_colsum32(q);
-        }
+        for (int k = 0; k < TC_UNITS; ++k) q[k] = da[k] * xn2;
+        g_w1[2] += warp_colsum16(q);
         tc_fence_before();
     }
     if (failed) {
@@ -323,33 +352,35 @@ __global__ void __launch_bounds__(TC_THREADS, 1) mlp_train_tc_kernel(const float
         mbar_wait_bounded(&S.bar[1], phase, TC_WAIT_POLLS);
     } else if (any_tile) {
         // ---- dW2: accumulator rows u (hi part) and 64 + u (lo part), summed
-        float acc[64];
-        tc_ld64(tmem, 128, acc);
+        float acc[TC_UNITS];
+        tc_ld16(tmem + ((uint32_t)(warp & 3) << 21) + 128u + (uint32_t)u0, acc);
+        tc_wait_ld();
         __syncthreads();   // every MMA has completed; the row tiles are free
         float* red = reinterpret_cast<float*>(S.a1k);   // [128][65] floats over a1k and dzk
 #pragma unroll
-        for (int v = 0; v < 64; ++v) red[tid * 65 + v] = acc[v];
+        for (int v = 0; v < TC_UNITS; ++v) red[rt * 65 + u0 + v] = acc[v];
         __syncthreads();
         for (int k = tid; k < MLP_H * MLP_H; k += TC_THREADS) {
             const int u = k >> 6, v = k & 63;
             atomicAdd(&grad[KNC_MLP_OFF_W2 + k], red[u * 65 + v] + red[(64 + u) * 65 + v]);
         }
+        if (grp == 0) {
 #pragma unroll
-        for (int o = 16; o > 0; o >>= 1) {
-            g_b3 += __shfl_xor_sync(0xffffffffu, g_b3, o);
-            l_sum += __shfl_xor_sync(0xffffffffu, l_sum, o);
+            for (int o = 16; o > 0; o >>= 1) {
+                g_b3 += __shfl_xor_sync(0xffffffffu, g_b3, o);
+                l_sum += __shfl_xor_sync(0xffffffffu, l_sum, o);
+            }
+            if (lane == 0) {
+                atomicAdd(&grad[KNC_MLP_OFF_B3], g_b3);
+                atomicAdd(loss_sum, l_sum);
+            }
         }
-        if (lane == 0) {
-            atomicAdd(&grad[KNC_MLP_OFF_B3], g_b3);
-            atomicAdd(loss_sum, l_sum);
-        }
-#pragma unroll
-        for (int hh = 0; hh < 2; ++hh) {
-            const int u = 32 * hh + lane;
-            atomicAdd(&grad[KNC_MLP_OFF_W3 + u], g_w3[hh]);
-            atomicAdd(&grad[KNC_MLP_OFF_B2 + u], g_b2[hh]);
-            atomicAdd(&grad[KNC_MLP_OFF_B1 + u], g_b1[hh]);
-            for (int k = 0; k < 3; ++k) atomicAdd(&grad[KNC_MLP_OFF_W1 + u * 3 + k], g_w1[k][hh]);
+        if (!(lane & 1)) {
+            const int u = u0 + (lane >> 1);
+            atomicAdd(&grad[KNC_MLP_OFF_W3 + u], g_w3);
+            atomicAdd(&grad[KNC_MLP_OFF_B2 + u], g_b2);
+            atomicAdd(&grad[KNC_MLP_OFF_B1 + u], g_b1);
+            for (int k = 0; k < 3; ++k) atomicAdd(&grad[KNC_MLP_OFF_W1 + u * 3 + k], g_w1[k]);
         }
     }
     tc_fence_before();
@@ -358,20 +389,26 @@ __global__ void __launch_bounds__(TC_THREADS, 1) mlp_train_tc_kernel(const float
         tc_fence_after();
         tc_dealloc(tmem, TC_TMEM_COLS);
     }
-}
-
-__global__ void adam_kernel(float* w, float* m, float* v, float* g, int n, float lr, float b1, float b2, float eps,
-                            float c1, float c2) {
-    const int k = blockIdx.x * blockDim.x + threadIdx.x;
-    if (k >= n) return;
-    const float gk = g[k];
-    g[k] = 0.f;
-    if (k >= KNC_MLP_OFF_XMEAN) return;   // input normalisation is fixed
-    const float mk = b1 * m[k] + (1.f - b1) * gk;
-    const float vk = b2 * v[k] + (1.f - b2) * gk * gk;
-    m[k] = mk;
-    v[k] = vk;
-    w[k] -= lr * (mk * c1) / (sqrtf(vk * c2) + eps);
+    // ---- the Adam step, by the CTA that adds its gradients last (it waits for
+    // nothing: the others have finished)
+    if (!adam.w) return;
+    __threadfence();
+    __syncthreads();
+    if (tid == 0) S.last = atomicAdd(adam.done, 1u) + 1u == gridDim.x ? 1u : 0u;
+    __syncthreads();
+    if (!S.last) return;
+    __threadfence();
+    if (tid == 0) *adam.done = 0u;
+    for (int k = tid; k < KNC_MLP_NUM_PARAMS; k += TC_THREADS) {
+        const float gk = __ldcg(&grad[k]);
+        grad[k] = 0.f;
+        if (k >= KNC_MLP_OFF_XMEAN) continue;   // input normalisation is fixed
+        const float mk = adam.b1 * adam.m[k] + (1.f - adam.b1) * gk;
+        const float vk = adam.b2 * adam.v[k] + (1.f - adam.b2) * gk * gk;
+        adam.m[k] = mk;
+        adam.v[k] = vk;
+        adam.w[k] -= adam.lr * (mk * adam.c1) / (sqrtf(vk * adam.c2) + adam.eps);
+    }
 }
 
 // Features and target of each pair, in FP32 exactly as the c2p kernels form them.
@@ -544,7 +581,7 @@ int knc_mlp_forward_backward(const float* weights, const float* x, const float* 
     CKR(cudaMemset(dl.p, 0, 4));
     mlp_train_tc_kernel<<<grid_for_rows(n), TC_THREADS, train_smem_bytes()>>>(
         (const float*)dw.p, (const float*)dx.p, (const float*)dy.p, n, n, 0ull, 1.0f / (float)n, (float*)dg.p,
-        (float*)dl.p, (float*)dp.p, (unsigned*)de.p);
+        (float*)dl.p, (float*)dp.p, (unsigned*)de.p, AdamArgs{});
     CKR(cudaGetLastError());
     unsigned err = 0;
     CKR(cudaMemcpy(&err, de.p, 4, cudaMemcpyDeviceToHost));
@@ -562,8 +599,8 @@ int knc_mlp_train(const double* pairs, int64_t n, float* weights, const knc_mlp_
     if (!pairs || n <= 0 || !weights || !tp || tp->batch <= 0 || tp->steps < 0) return KNC_ERR_INVALID_ARGUMENT;
     CKR(configure_train());
     DevBuf dpairs, dx, dy, dw, dm, dv, dg, dl, de;
-    CKR(cudaMalloc(&de.p, 4));
-    CKR(cudaMemset(de.p, 0, 4));
+    CKR(cudaMalloc(&de.p, 8));      // error word, count of finished CTAs
+    CKR(cudaMemset(de.p, 0, 8));
     CKR(cudaMalloc(&dpairs.p, (size_t)n * 8 * sizeof(double)));
     CKR(cudaMalloc(&dx.p, (size_t)n * 12));
     CKR(cudaMalloc(&dy.p, (size_t)n * 4));
@@ -581,13 +618,14 @@ int knc_mlp_train(const double* pairs, int64_t n, float* weights, const knc_mlp_
         const int64_t m = std::min<int64_t>(n, 1 << 18);
         std::vector<float> xs((size_t)m * 3);
         CKR(cudaMemcpy(xs.data(), dx.p, (size_t)m * 12, cudaMemcpyDeviceToHost));
-        for (int k = 0; k < 3; ++k) {
-            double s = 0, s2 = 0;
-            for (int64_t r = 0; r < m; ++r) {
-                s += xs[r * 3 + k];
-                s2 += (double)xs[r * 3 + k] * xs[r * 3 + k];
+        double s[3] = {0, 0, 0}, s2[3] = {0, 0, 0};   // the columns' chains of additions side by side
+        for (int64_t r = 0; r < m; ++r)
+            for (int k = 0; k < 3; ++k) {
+                s[k] += xs[r * 3 + k];
+                s2[k] += (double)xs[r * 3 + k] * xs[r * 3 + k];
             }
-            const double mean = s / m, var = std::max(s2 / m - mean * mean, 1e-12);
+        for (int k = 0; k < 3; ++k) {
+            const double mean = s[k] / m, var = std::max(s2[k] / m - mean * mean, 1e-12);
             w[KNC_MLP_OFF_XMEAN + k] = (float)mean;
             w[KNC_MLP_OFF_XSCALE + k] = (float)(1.0 / std::sqrt(var));
         }
@@ -604,17 +642,16 @@ int knc_mlp_train(const double* pairs, int64_t n, float* weights, const knc_mlp_
     double p1 = 1.0, p2 = 1.0;
     for (int64_t step = 0; step < tp->steps; ++step) {
         const uint64_t seed = splitmix64((tp->seed ? tp->seed : 1ull) + (uint64_t)step * 0x9E3779B97F4A7C15ull) | 1ull;
-        mlp_train_tc_kernel<<<grid, TC_THREADS, train_smem_bytes()>>>(
-            (const float*)dw.p, (const float*)dx.p, (const float*)dy.p, n, batch, seed, 1.0f / (float)batch,
-            (float*)dg.p, (float*)dl.p, nullptr, (unsigned*)de.p);
         p1 *= b1;
         p2 *= b2;
         // learning-rate decay: cosine over the run to 5 % of the initial rate
         const double frac = tp->steps > 1 ? (double)step / (double)(tp->steps - 1) : 1.0;
         const float lr = (float)(tp->lr * (0.05 + 0.95 * 0.5 * (1.0 + std::cos(3.14159265358979 * frac))));
-        adam_kernel<<<(KNC_MLP_NUM_PARAMS + 255) / 256, 256>>>((float*)dw.p, (float*)dm.p, (float*)dv.p,
-                                                               (float*)dg.p, KNC_MLP_NUM_PARAMS, lr, b1, b2, eps,
-                                                               (float)(1.0 / (1.0 - p1)), (float)(1.0 / (1.0 - p2)));
+        const AdamArgs adam = {(float*)dw.p, (float*)dm.p, (float*)dv.p, (unsigned*)de.p + 1, lr, b1, b2, eps,
+                               (float)(1.0 / (1.0 - p1)), (float)(1.0 / (1.0 - p2))};
+        mlp_train_tc_kernel<<<grid, TC_THREADS, train_smem_bytes()>>>(
+            (const float*)dw.p, (const float*)dx.p, (const float*)dy.p, n, batch, seed, 1.0f / (float)batch,
+            (float*)dg.p, (float*)dl.p, nullptr, (unsigned*)de.p, adam);
     }
     CKR(cudaGetLastError());
     // final loss over (up to) the first 1M rows
@@ -622,7 +659,7 @@ int knc_mlp_train(const double* pairs, int64_t n, float* weights, const knc_mlp_
     CKR(cudaMemset(dl.p, 0, 4));
     mlp_train_tc_kernel<<<grid_for_rows(ev), TC_THREADS, train_smem_bytes()>>>(
         (const float*)dw.p, (const float*)dx.p, (const float*)dy.p, n, ev, 0ull, 1.0f / (float)ev, (float*)dg.p,
-        (float*)dl.p, nullptr, (unsigned*)de.p);
+        (float*)dl.p, nullptr, (unsigned*)de.p, AdamArgs{});
     CKR(cudaGetLastError());
     unsigned err = 0;
     CKR(cudaMemcpy(&err, de.p, 4, cudaMemcpyDeviceToHost));

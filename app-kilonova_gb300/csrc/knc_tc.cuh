@@ -85,17 +85,4 @@ __device__ __forceinline__ void tc_ld16(uint32_t taddr, float (&v)[16]) {
 
 __device__ __forceinline__ void tc_wait_ld() { asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory"); }
 
-// 64 FP32 columns starting at column `col` of this warp's lanes.
-__device__ __forceinline__ void tc_ld64(uint32_t tmem, int col, float (&v)[64]) {
-    const uint32_t base = tmem + ((uint32_t)(threadIdx.x & ~31u) << 16) + (uint32_t)col;
-    float t[16];
-#pragma unroll
-    for (int c = 0; c < 4; ++c) {
-        tc_ld16(base + 16u * c, t);
-        tc_wait_ld();
-#pragma unroll
-        for (int k = 0; k < 16; ++k) v[16 * c + k] = t[k];
-    }
-}
-
 }  // namespace knc
