@@ -102,4 +102,21 @@ __device__ __forceinline__ double half_exact(double x) {
     return x * 0.5;
 }
 
+// The same without an FP64 instruction: exact for normal numbers above the
+// smallest, zeros, infinities and NaNs; half_odd says whether x is none of them.
+// The words come through asm: the compiler turns integer tests on a double's
+// bits into FP64 comparisons.
+__device__ __forceinline__ double half_normal(double x) {
+    uint32_t hi, lo;
+    asm("mov.b64 {%0, %1}, %2;" : "=r"(lo), "=r"(hi) : "d"(x));
+    return __hiloint2double((int)((hi & 0x7fffffffu) - (2u << 20) < (2045u << 20) ? hi - (1u << 20) : hi), (int)lo);
+}
+__device__ __forceinline__ bool half_odd(double x) {
+    uint32_t hi, lo;
+    asm("mov.b64 {%0, %1}, %2;" : "=r"(lo), "=r"(hi) : "d"(x));
+    const uint32_t h = hi & 0x7fffffffu;
+    return h < (2u << 20) && (h | lo) != 0u;
+}
+static __device__ __noinline__ double half_subnormal(double x) { return x * 0.5; }
+
 }  // namespace knc

@@ -831,8 +831,21 @@ __device__ __forceinline__ void update_strip(const StageArgs& a, const int4 it, 
             }
             if (U0) {
                 if (MIXED && a.avg_half) {
+                    bool odd = false;
 #pragma unroll
-                    for (int q = 0; q < NFIELD; ++q) res[q] = half_exact(res[q] + U0[q * n + z]);
+                    for (int q = 0; q < NFIELD; ++q) {
+                        res[q] += U0[q * n + z];
+                        odd = odd || half_odd(res[q]);
+                    }
+                    if (odd) {
+                        // (out of line: in line the products would be issued
+                        // under a predicate for every row)
+#pragma unroll
+                        for (int q = 0; q < NFIELD; ++q) res[q] = half_subnormal(res[q]);
+                    } else {
+#pragma unroll
+                        for (int q = 0; q < NFIELD; ++q) res[q] = half_normal(res[q]);
+                    }
                 } else {
 #pragma unroll
                     for (int q = 0; q < NFIELD; ++q) res[q] = res[q] * a.w1 + U0[q * n + z] * a.bf;
