@@ -242,14 +242,27 @@ constexpr int STREAM_STRIP_ROWS = 4;
 // 5.22 (8 rows throughout) -> 4.78 ms, over 1, 2, 3: 4.74, 4.94, 5.00;
 // Newtonian sphere 4.12 -> 3.83 ms. Grids under 16 rows per partition take 2
 // throughout (450 x 230, RK3: 2 rows 1.10 ms, 3 to 4 1.18, 1 1.36; 256 x 128:
-// 2 rows 235 us, 1 229, 3 267).
+// 2 rows 235 us, 1 229, 3 267). Grids under 8 rows per partition take tiles
+// instead (`tiles`): rows per partition, items and tiles in us: 0.4 (Newtonian
+// sphere) 283, 213; 5.9 (RK3 HLLC) 995, 942; 10 (wind) 1037, 1009, (sphere)
+// 984, 986; 20 (sphere) 1650, 1743.
 constexpr double F64_ROWS_OVER = 1.5, F64_ROWS_LEAST = 2.0, F64_ROWS_MOST = 16.0, F64_ROWS_SMALL_GRID = 16.0;
+constexpr double F64_TILE_GRID = 8.0;
 
-std::vector<int4> f64_items(const std::vector<std::pair<int64_t, int64_t>>& shapes, int slot0, int sms) {
+std::vector<int4> f64_items(const std::vector<std::pair<int64_t, int64_t>>& shapes, int slot0, int sms, bool& tiles) {
     double left = 0.0;   // rows of 32 columns left, per SM partition
     for (const auto& s : shapes) left += (double)(s.first * ((s.second + TILE_Q - 1) / TILE_Q)) / (4.0 * sms);
     const double most = left < F64_ROWS_SMALL_GRID ? F64_ROWS_LEAST : F64_ROWS_MOST;
     std::vector<int4> items;
+    tiles = left < F64_TILE_GRID;
+    if (tiles) {
+        for (size_t k = 0; k < shapes.size(); ++k)
+            for (int64_t i0 = 0; i0 < shapes[k].first; i0 += 2)
+                for (int64_t j0 = 0; j0 < shapes[k].second; j0 += TILE64_COLS)
+                    items.push_back(make_int4(slot0 + (int)k, (int)i0, (int)j0,
+                                              (int)std::min<int64_t>(2, shapes[k].first - i0)));
+        return items;
+    }
     for (size_t k = 0; k < shapes.size(); ++k) {
         const int64_t nr = shapes[k].first, nq = shapes[k].second, cols = (nq + TILE_Q - 1) / TILE_Q;
         for (int64_t i0 = 0; i0 < nr;) {
@@ -278,6 +291,7 @@ struct Layout {
     int uform = -1;
     int list_cols = 0;          // columns of a strip: 32 for the FP64 update's items, else STRIP_OUT
     bool list_auto = false;     // item rows by f64_items
+    bool f64_tiles = false;     // the utiles are tiles of TILE64_COLS columns
     int64_t nzones = 0;         // zones of the block set
     TmaMaps* d_tmaps = nullptr; // tensor maps per slot (tiles of `utr` rows), when every block allows them
     int tmaps_cap = 0;
@@ -315,6 +329,7 @@ struct Layout {
     std::vector<int> sc_tile_off;        // [G + 1]
     std::vector<int> sc_own_tiles;       // [G]
     std::vector<int> sc_strip_off;       // [G S + 1]: chunk k, stage s at k S + s
+    std::vector<char> sc_tiles64;        // per chunk: its FP64 update items are tiles
     std::vector<int64_t> sc_up;          // [G + 1]: zones each chunk's upload covers
     DevBlock* d_sc_table = nullptr;
     int sc_table_cap = 0;
@@ -781,7 +796,9 @@ int rebuild_table(knc_ctx* c) {
     if (rows_auto) {
         std::vector<std::pair<int64_t, int64_t>> shapes;
         for (const BlockH* b : order) shapes.push_back({b->nr, b->nq});
-        utiles = f64_items(shapes, 0, c->sms);
+        utiles = f64_items(shapes, 0, c->sms, L(c).f64_tiles);
+    } else {
+        L(c).f64_tiles = false;
     }
     L(c).tile_off.push_back((int)tiles.size());
     L(c).utile_off.push_back((int)utiles.size());
@@ -1035,6 +1052,7 @@ StageArgs base_args(knc_ctx* c) {
     a.utr = L(c).utr;
     a.tma = c->uform == KNC_UPDATE_TILE_TMA && L(c).tma_ok ? 1 : 0;
     a.tmaps = L(c).tma_ok ? L(c).d_tmaps : nullptr;
+    a.f64_tiles = L(c).f64_tiles ? 1 : 0;
     a.strips = c->uform == KNC_UPDATE_STRIP ? L(c).d_strips : nullptr;
     a.nstrips = c->uform == KNC_UPDATE_STRIP ? L(c).nstrips : 0;
     a.strip_ctas = c->ctas_per_sm >= 4 && c->ctas_per_sm <= 6 ? c->ctas_per_sm : 4;
@@ -2361,13 +2379,16 @@ int build_chunks(knc_ctx* c, int S) {
     // its shadows' rows that stage updates
     std::vector<int4> strips;
     l.sc_strip_off.clear();
+    l.sc_tiles64.clear();
     for (int k = 0; k < G; ++k)
         for (int s = 0; s < S; ++s) {
             l.sc_strip_off.push_back((int)strips.size());
             if (l.list_cols == TILE_Q) {   // the FP64 update's items
                 std::vector<std::pair<int64_t, int64_t>> shapes;
                 for (int b = cb[k]; b < cb[k + 1]; ++b) shapes.push_back({l.tab_h[b].nr, l.tab_h[b].nq});
-                const std::vector<int4> items = f64_items(shapes, cb[k], c->sms);
+                bool tiles = false;
+                const std::vector<int4> items = f64_items(shapes, cb[k], c->sms, tiles);
+                if (s == 0) l.sc_tiles64.push_back(tiles ? 1 : 0);
                 strips.insert(strips.end(), items.begin(), items.end());
             } else {
                 strips.insert(strips.end(), l.sstrips_h.begin() + l.sstrip_off[cb[k]],
@@ -2378,6 +2399,12 @@ int build_chunks(knc_ctx* c, int S) {
             for (int n : of_chunk[k]) {
                 const Shadow& x = sh[n];
                 const int i0 = x.upper ? 0 : 2 * s + 2;
+                if (l.list_cols == TILE_Q && l.sc_tiles64[k]) {
+                    for (int r = 0; r < rows; r += 2)   // (an even number of rows)
+                        for (int j0 = 0; j0 < tab[x.src].nq; j0 += TILE64_COLS)
+                            strips.push_back(make_int4(nb + n, i0 + r, j0, 2));
+                    continue;
+                }
                 for (int j0 = 0; j0 < tab[x.src].nq; j0 += l.list_cols)
                     strips.push_back(make_int4(nb + n, i0, j0, rows));
             }
@@ -2540,6 +2567,7 @@ int stream_step(knc_ctx* c, double dt, const double* hc_in, const double* hs_in,
             // the tuned form (every form gives the same state)
             y.strips = lay.d_sc_strips + lay.sc_strip_off[k * S + s];
             y.nstrips = lay.sc_strip_off[k * S + s + 1] - lay.sc_strip_off[k * S + s];
+            y.f64_tiles = lay.list_cols == TILE_Q ? lay.sc_tiles64[k] : 0;
             y.tma = 0;
             // chunks run side by side: no shared list (each strip checks its
             // own stencil and updates its zones with FP64 faces itself)

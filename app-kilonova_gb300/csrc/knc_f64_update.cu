@@ -127,6 +127,58 @@ __device__ __forceinline__ void edges64(const StageArgs& a, const PhysT<double>&
     for (int q = 0; q < NFIELD; ++q) E.flux[q][lane] = f[q];
 }
 
+// Sources, conserved update and RK average of zone (i, j) with primitive P0:
+// radial fluxes Flo, Fhi, polar flux difference D.
+template <bool SRHD>
+__device__ __forceinline__ void update_zone64(const StageArgs& a, const PhysT<double>& ph, const DevBlock& B, int i,
+                                              int j, const double* P0, const double* Flo, const double* Fhi,
+                                              const double* D, bool one_d, double dt) {
+    const int64_t n = (int64_t)B.nr * B.nq, z = (int64_t)i * B.nq + j;
+    const double* Uin = B.buf[a.sel_in];
+    double* Uout = B.buf[a.sel_out];
+    double s1, s2, res[NFIELD];
+    const double dV = B.dv[z];
+    sources64<SRHD>(ph, P0, B.rc[i], B.cot[j], s1, s2);
+    s1 = (SRHD ? s1 * a.cflux : s1) * dV;
+    s2 = (SRHD ? s2 * a.cflux : s2) * dV;
+#pragma unroll
+    for (int q = 0; q < NFIELD; ++q) {
+        const double R = Fhi[q] - Flo[q];
+        double du;
+        // (S - dF_r - dF_q) dt; without a source the exact negative of (dF_r + dF_q) dt
+        if (q == 1 || q == 2) {
+            const double sc = q == 1 ? s1 : s2;
+            du = (one_d ? sc - R : sc - R - D[q]) * dt;
+        } else {
+            du = -((one_d ? R : R + D[q]) * dt);
+        }
+        res[q] = Uin[q * n + z] + du;
+    }
+    if (a.sel_base >= 0) {
+        // res w1 + U0 b
+        const double* U0 = B.buf[a.sel_base];
+        bool odd = false;
+        double u0[NFIELD];
+#pragma unroll
+        for (int q = 0; q < NFIELD; ++q) {
+            u0[q] = U0[q * n + z];
+            odd = odd || odd_average(res[q]) || odd_average(u0[q]);
+        }
+        if (odd || !(a.avg_half || a.w1 == 0.25)) {
+#pragma unroll
+            for (int q = 0; q < NFIELD; ++q) res[q] = res[q] * a.w1 + u0[q] * a.bf;
+        } else if (a.avg_half) {
+#pragma unroll
+            for (int q = 0; q < NFIELD; ++q) res[q] = half64(res[q] + u0[q]);
+        } else {
+#pragma unroll
+            for (int q = 0; q < NFIELD; ++q) res[q] = __fma_rn(res[q], 0.25, u0[q] * a.bf);
+        }
+    }
+#pragma unroll
+    for (int q = 0; q < NFIELD; ++q) Uout[q * n + z] = res[q];
+}
+
 template <bool SRHD, bool HLLC>
 __device__ __forceinline__ void update_rows64(const StageArgs& a, const PhysT<double>& ph, const int4 it, Edge64& E) {
     const unsigned full = 0xffffffffu;
@@ -137,12 +189,9 @@ __device__ __forceinline__ void update_rows64(const StageArgs& a, const PhysT<do
     const bool jin = j < nq;
     const bool one_d = a.one_dimensional != 0;
     const double* P = reinterpret_cast<const double*>(B.P);
-    const int64_t pn = (int64_t)(nr + 4) * nq, n = (int64_t)nr * nq;
+    const int64_t pn = (int64_t)(nr + 4) * nq;
     const double th = ph.theta, c = a.cflux;
     const double dt = stage_dt<double>(a);
-    const double* Uin = B.buf[a.sel_in];
-    double* Uout = B.buf[a.sel_out];
-    const double* U0 = a.sel_base >= 0 ? B.buf[a.sel_base] : nullptr;
     const bool pedge = j <= 0 || j >= nq - 1;   // zero polar slope on the block's first and last column
     // the column a first or last lane reads beyond the warp's
     const int je = lane == 0 ? j0 - 1 : j0 + 32;
@@ -175,7 +224,7 @@ __device__ __forceinline__ void update_rows64(const StageArgs& a, const PhysT<do
     }
     for (int s = 0; s < rows; ++s) {
         const int i = i0 + s;
-        const int64_t z = (int64_t)i * nq + j, o = z + 2 * (int64_t)nq;
+        const int64_t o = (int64_t)(i + 2) * nq + j;
         double P2[NFIELD];
         load_row64(P, pn, o + 2 * (int64_t)nq, jin, P2);
         // ---- polar faces j (own) and j + 1 (the next lane's)
@@ -225,49 +274,7 @@ __device__ __forceinline__ void update_rows64(const StageArgs& a, const PhysT<do
                 through_area<SRHD>(Fhi, c, B.ar[(int64_t)(i + 1) * nq + j]);
             }
         }
-        // ---- sources, conserved update, RK average of zone (i, j)
-        if (jin) {
-            double s1, s2, res[NFIELD];
-            const double dV = B.dv[z];
-            sources64<SRHD>(ph, P0, B.rc[i], B.cot[j], s1, s2);
-            s1 = (SRHD ? s1 * c : s1) * dV;
-            s2 = (SRHD ? s2 * c : s2) * dV;
-#pragma unroll
-            for (int q = 0; q < NFIELD; ++q) {
-                const double R = Fhi[q] - Flo[q];
-                double du;
-                // (S - dF_r - dF_q) dt; without a source the exact negative of (dF_r + dF_q) dt
-                if (q == 1 || q == 2) {
-                    const double sc = q == 1 ? s1 : s2;
-                    du = (one_d ? sc - R : sc - R - D[q]) * dt;
-                } else {
-                    du = -((one_d ? R : R + D[q]) * dt);
-                }
-                res[q] = Uin[q * n + z] + du;
-            }
-            if (U0) {
-                // res w1 + U0 b
-                bool odd = false;
-                double u0[NFIELD];
-#pragma unroll
-                for (int q = 0; q < NFIELD; ++q) {
-                    u0[q] = U0[q * n + z];
-                    odd = odd || odd_average(res[q]) || odd_average(u0[q]);
-                }
-                if (odd || !(a.avg_half || a.w1 == 0.25)) {
-#pragma unroll
-                    for (int q = 0; q < NFIELD; ++q) res[q] = res[q] * a.w1 + u0[q] * a.bf;
-                } else if (a.avg_half) {
-#pragma unroll
-                    for (int q = 0; q < NFIELD; ++q) res[q] = half64(res[q] + u0[q]);
-                } else {
-#pragma unroll
-                    for (int q = 0; q < NFIELD; ++q) res[q] = __fma_rn(res[q], 0.25, u0[q] * a.bf);
-                }
-            }
-#pragma unroll
-            for (int q = 0; q < NFIELD; ++q) Uout[q * n + z] = res[q];
-        }
+        if (jin) update_zone64<SRHD>(a, ph, B, i, j, P0, Flo, Fhi, D, one_d, dt);
 #pragma unroll
         for (int q = 0; q < NFIELD; ++q) {
             Flo[q] = Fhi[q];
@@ -291,10 +298,105 @@ __global__ void __launch_bounds__(ROWS64_WARPS * 32, 3)
         update_rows64<SRHD, HLLC>(a, ph, items[k], sE[w]);
 }
 
+// ---- small grids ------------------------------------------------------------------
+// A march does an item's faces one after the other: with a few rows per SM
+// partition its length, not the FP64 pipe, sets the kernel's time. Here a CTA of
+// 4 warps takes a tile of at most TILE64_ROWS rows x 31 columns and its warps
+// claim face passes, the rows' 32 polar faces first, then the rows + 1 rows of
+// radial faces; fluxes meet in shared memory, then a warp per row updates it.
+// Slopes are formed by the faces on both of their sides (25 FP64 instructions
+// more per face than in the march), with the same roundings.
+constexpr int TILE64_ROWS = 2;
+
+struct Tile64 {
+    double P[NFIELD][TILE64_ROWS + 4][TILE64_COLS + 4];
+    double Fr[NFIELD][TILE64_ROWS + 1][32];
+    double Fq[NFIELD][TILE64_ROWS][32];
+    unsigned claim;
+};
+
+template <bool SRHD, bool HLLC>
+__global__ void __launch_bounds__(ROWS64_WARPS * 32, 3)
+    update_tile64_kernel(const __grid_constant__ StageArgs a, const int4* __restrict__ items) {
+    __shared__ Tile64 T;
+    if (*(volatile unsigned long long*)&a.status->err_key != NO_ERROR) return;
+    const PhysT<double> ph = make_phys<double>(a);
+    const int4 it = items[blockIdx.x];
+    const DevBlock& B = a.blocks[it.x];
+    const int nr = B.nr, nq = B.nq, i0 = it.y, j0 = it.z, rows = it.w;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const bool one_d = a.one_dimensional != 0;
+    const double th = ph.theta;
+    {
+        const double* P = reinterpret_cast<const double*>(B.P);
+        const int64_t pn = (int64_t)(nr + 4) * nq;
+        constexpr int PC = TILE64_COLS + 4;
+        for (int k = threadIdx.x; k < (rows + 4) * PC; k += ROWS64_WARPS * 32) {
+            const int r = k / PC, c = k - r * PC, j = j0 - 2 + c;
+            const bool ok = j >= 0 && j < nq;
+            const int64_t o = (int64_t)(i0 + r) * nq + j;   // padded row i0 is zone row i0 - 2
+#pragma unroll
+            for (int q = 0; q < NFIELD; ++q) T.P[q][r][c] = ok ? P[q * pn + o] : 0.0;
+        }
+        if (threadIdx.x == 0) T.claim = ROWS64_WARPS;
+    }
+    __syncthreads();
+    const unsigned polar = one_d ? 0u : (unsigned)rows, passes = polar + (unsigned)rows + 1u;
+    const int j = j0 + lane;
+    // A warp's first pass is rotated with the CTA: a warp stays on its SM
+    // partition, and the polar faces cost more than supersonic radial ones.
+    unsigned p = (warp + blockIdx.x) % ROWS64_WARPS;
+    while (p < passes) {
+        const bool radial = p >= polar;
+        const int r = (int)(radial ? p - polar : p);   // radial face i0 + r, or row i0 + r
+        const bool exists = radial ? lane < TILE64_COLS && j < nq : j > 0 && j < nq;
+        double f[NFIELD] = {0.0, 0.0, 0.0, 0.0, 0.0};
+        if (exists) {
+            // the face lies between the second and third of its four zones
+            const bool zl = !radial && j - 1 == 0, zr = !radial && j == nq - 1;   // zero polar slope on the edge columns
+            double pl[NFIELD], pr[NFIELD];
+#pragma unroll
+            for (int q = 0; q < NFIELD; ++q) {
+                const double* s = radial ? &T.P[q][r][lane + 2] : &T.P[q][r + 2][lane];
+                const int st = radial ? TILE64_COLS + 4 : 1;
+                const double s0 = s[0], s1 = s[st], s2 = s[2 * st], s3 = s[3 * st];
+                const double mid = th * (s2 - s1);
+                pl[q] = s1 + (zl ? 0.0 : half_slope64(th * (s1 - s0), s2 - s0, mid));
+                pr[q] = s2 - (zr ? 0.0 : half_slope64(mid, s3 - s1, th * (s3 - s2)));
+            }
+            item_face<SRHD, HLLC>(a, ph, pl, pr, radial ? 0 : 1, f);
+            through_area<SRHD>(f, a.cflux, radial ? B.ar[(int64_t)(i0 + r) * nq + j] : B.aq[(int64_t)(i0 + r) * (nq + 1) + j]);
+        }
+#pragma unroll
+        for (int q = 0; q < NFIELD; ++q) (radial ? T.Fr[q][r] : T.Fq[q][r])[lane] = f[q];
+        if (lane == 0) p = atomicAdd(&T.claim, 1u);
+        p = __shfl_sync(0xffffffffu, p, 0);
+    }
+    __syncthreads();
+    if (warp < rows && lane < TILE64_COLS && j < nq) {
+        const int r = warp;
+        double P0[NFIELD], lo[NFIELD], hi[NFIELD], D[NFIELD];
+#pragma unroll
+        for (int q = 0; q < NFIELD; ++q) {
+            P0[q] = T.P[q][r + 2][lane + 2];
+            lo[q] = T.Fr[q][r][lane];
+            hi[q] = T.Fr[q][r + 1][lane];
+            D[q] = one_d ? 0.0 : T.Fq[q][r][lane + 1] - T.Fq[q][r][lane];
+        }
+        update_zone64<SRHD>(a, ph, B, i0 + r, j, P0, lo, hi, D, one_d, stage_dt<double>(a));
+    }
+}
+
 cudaError_t launch_update_f64(const StageArgs& a, cudaStream_t s) {
     const int4* items = a.strips ? a.strips : a.utiles;
     const int n = a.strips ? a.nstrips : a.nutiles;
     if (n <= 0) return cudaSuccess;
+    if (a.f64_tiles) {
+        auto k = a.srhd ? (a.hllc ? update_tile64_kernel<true, true> : update_tile64_kernel<true, false>)
+                        : (a.hllc ? update_tile64_kernel<false, true> : update_tile64_kernel<false, false>);
+        k<<<n, ROWS64_WARPS * 32, 0, s>>>(a, items);
+        return cudaGetLastError();
+    }
     const int grid = (n + ROWS64_WARPS - 1) / ROWS64_WARPS;
     auto k = a.srhd ? (a.hllc ? update_rows64_kernel<true, true> : update_rows64_kernel<true, false>)
                     : (a.hllc ? update_rows64_kernel<false, true> : update_rows64_kernel<false, false>);

@@ -31,6 +31,7 @@ constexpr int TILE_THREADS = TILE_R * TILE_Q;
 constexpr int NFIELD = 5;
 constexpr int STRIP_OUT = TILE_Q - 4;   // output columns of a warp strip (2 halo lanes each side)
 constexpr int STRIP_WARPS = 4;          // independent strips per CTA
+constexpr int TILE64_COLS = 31;         // columns of an FP64 update tile: their 32 polar faces fill a warp
 
 struct DevBlock {
     double* buf[2];        // [5][nr][nq] state ping/pong
@@ -120,6 +121,7 @@ struct StageArgs {
     int32_t tma;            // mixed update: stage tiles with tensor copies (tmaps valid)
     const int4* strips;     // {slot, i0, j0, rows}: warp strips of the strip form, or null
     int32_t nstrips;
+    int32_t f64_tiles;      // FP64 update: the items are tiles of TILE64_COLS columns (small grids)
     int32_t strip_ctas;     // strip form: CTAs per SM the kernel is built for (4, 5 or 6)
     int32_t fused_wide;     // fused deferring stage: one CTA of 20 warps per SM
     // adaptive dt found on the device (the fold's first recovery reduces
@@ -250,7 +252,8 @@ cudaError_t configure_kernels();
 cudaError_t launch_init_f64(const InitArgs& a, int ntiles, cudaStream_t s);
 cudaError_t launch_c2p_f64(const StageArgs& a, cudaStream_t s);
 // The FP64 update over the items {slot, i0, j0, rows <= 32} of a.strips (or
-// a.utiles), 32 columns each (knc_f64_update.cu).
+// a.utiles), 32 columns each, or tiles of at most 2 rows x TILE64_COLS columns
+// (a.f64_tiles) (knc_f64_update.cu).
 cudaError_t launch_update_f64(const StageArgs& a, cudaStream_t s);
 cudaError_t launch_ghost_f64(const GhostArgs& a, cudaStream_t s);
 cudaError_t launch_ghost_mixed(const GhostArgs& a, cudaStream_t s);
