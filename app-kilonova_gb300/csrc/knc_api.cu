@@ -1431,17 +1431,8 @@ int check_status(knc_ctx* c) {
 int reset_status(knc_ctx* c, bool keep_stats) {
     DevStatus* d = c->d_status;
     if (keep_stats) {
-        // stream-ordered field writes, no round trip: the error key and dt
-        // minimum to all-ones, the barrier and deferral counters to zero
-        CK(cudaMemsetAsync(&d->err_key, 0xff, sizeof(d->err_key), c->stream));
-        CK(cudaMemsetAsync(&d->err_sel, 0, sizeof(d->err_sel), c->stream));
-        CK(cudaMemsetAsync(&d->dt_bits, 0xff, sizeof(d->dt_bits), c->stream));
-        CK(cudaMemsetAsync(&d->bar_count, 0, sizeof(d->bar_count) + sizeof(d->bar_abort), c->stream));
-        CK(cudaMemsetAsync(d->high_count, 0, sizeof(d->high_count), c->stream));
-        CK(cudaMemsetAsync(d->hp_count, 0, sizeof(d->hp_count) + sizeof(d->hp_claim), c->stream));
-        // the fused deferring stage's item counter: a launch whose grid
-        // barrier gave up may leave it counting
-        CK(cudaMemsetAsync(&d->item_claim, 0, sizeof(d->item_claim), c->stream));
+        // one stream-ordered launch, no round trip
+        CK(launch_reset_status(d, c->stream));
     } else {
         DevStatus s;
         std::memset(&s, 0, sizeof(s));

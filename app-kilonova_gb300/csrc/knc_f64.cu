@@ -274,6 +274,26 @@ __global__ void products_kernel(const double* __restrict__ P, const double* __re
 }
 
 // ---- launchers ---------------------------------------------------------------
+__global__ void reset_status_kernel(DevStatus* d) {
+    d->err_key = NO_ERROR;
+    d->err_sel = 0;
+    d->dt_bits = ~0ull;
+    d->bar_count = 0ull;
+    d->bar_abort = 0;
+    // the counters of a launch whose grid barrier gave up too
+    for (int k = 0; k < 2; ++k) {
+        d->high_count[k] = 0u;
+        d->hp_count[k] = 0u;
+        d->hp_claim[k] = 0u;
+    }
+    d->item_claim = 0u;
+}
+
+cudaError_t launch_reset_status(DevStatus* d, cudaStream_t s) {
+    reset_status_kernel<<<1, 1, 0, s>>>(d);
+    return cudaGetLastError();
+}
+
 cudaError_t launch_products(const void* P, const double* U, double* prim, double* scalar, int64_t nr, int64_t nq,
                             cudaStream_t s) {
     const int64_t n = nr * nq;

@@ -250,6 +250,9 @@ void host_block_volumes(const knc_mesh_params& mesh, int32_t index, std::vector<
 // Set the kernels' shared-memory attributes once, before any launch or capture.
 cudaError_t configure_kernels();
 cudaError_t launch_init_f64(const InitArgs& a, int ntiles, cudaStream_t s);
+// The status word at the start of a call: error key and dt minimum to
+// all-ones, barrier, list and claim counters to zero; the statistics stay.
+cudaError_t launch_reset_status(DevStatus* d, cudaStream_t s);
 cudaError_t launch_c2p_f64(const StageArgs& a, cudaStream_t s);
 // The FP64 update over the items {slot, i0, j0, rows <= 32} of a.strips (or
 // a.utiles), 32 columns each, or tiles of at most 2 rows x TILE64_COLS columns
