@@ -231,6 +231,9 @@ void free_block(BlockH& b) {
 // 1.358, 1.379 ms).
 constexpr int STREAM_STRIP_ROWS = 4;
 
+// Strips per SM partition that a small grid's mixed update is spread to.
+constexpr int64_t MIXED_STRIPS = 2;
+
 // The FP64 update's items {slot, i0, j0, rows} (32 columns each,
 // knc_f64_update.cu) of the blocks slot0, slot0 + 1, ... with the given (nr,
 // nq), where the caller has not chosen their rows. An item costs about one
@@ -689,6 +692,15 @@ int rebuild_table(knc_ctx* c) {
         L(c).list_cols == cols && L(c).list_auto == rows_auto)
         return KNC_OK;
     const int64_t item_rows = rows64 ? std::min<int64_t>(c->utr, 32) : c->utr;
+    // Warp strips are utr rows high at most: where that would leave the mixed
+    // stage fewer than MIXED_STRIPS strips per SM partition, lower ones (a strip
+    // is a latency chain along its rows).
+    int64_t strip_rows = item_rows;
+    if (!rows64 && !c->fused) {
+        int64_t total = 0;
+        for (auto& kv : c->blocks) total += kv.second.nr * ((kv.second.nq + cols - 1) / cols);
+        strip_rows = std::min(strip_rows, std::max<int64_t>(1, total / (MIXED_STRIPS * 4 * c->sms)));
+    }
     L(c).list_cols = cols;
     L(c).list_auto = rows_auto;
     const int nb = (int)c->blocks.size();
@@ -773,7 +785,7 @@ int rebuild_table(knc_ctx* c) {
         if (c->uform == KNC_UPDATE_STRIP) {
             // ceil(nr / utr) strips per column, their heights as even as
             // whole rows allow (64 rows at utr 13: 13, 13, 13, 13, 12)
-            const int64_t per = (b.nr + item_rows - 1) / item_rows;
+            const int64_t per = (b.nr + strip_rows - 1) / strip_rows;
             for (int64_t j0 = 0; j0 < b.nq; j0 += cols)
                 for (int64_t k = 0, i0 = 0; k < per; ++k) {
                     const int64_t rows = b.nr / per + (k < b.nr % per ? 1 : 0);

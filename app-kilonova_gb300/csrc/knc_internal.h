@@ -172,6 +172,7 @@ struct StageArgs {
     unsigned* high_count;       // this stage's count (status word, by stage parity)
     unsigned* high_count_next;  // the next stage's, cleared by the dense pass
     unsigned high_cap;          // entries a.high holds
+    int32_t row_split;          // row-walking recovery: warps per recovery tile (1, 2, 4 or 8)
     int32_t avg_half;       // w1 == bf == 1/2 (the RK2 average, halved exactly on the integer pipe)
     const float* mlp;       // packed MLP weights (device) or null
     DevStatus* status;

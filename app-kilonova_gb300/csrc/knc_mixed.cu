@@ -395,18 +395,18 @@ __device__ __forceinline__ void cp_async_wait() {
     asm volatile("cp.async.wait_group %0;\n" ::"n"(N) : "memory");
 }
 
-// One recovery tile t = {slot, i0, j0, -} walked by the calling warp: its
-// TILE_R rows of 32 zones, each lane's column of the next rows copied ahead
-// into the warp's staging slots sUw. Zones that need the FP64 recovery go to
+// Rows i0 .. i0 + most - 1 (as far as the block goes) of a recovery tile t =
+// {slot, i0, j0, -} walked by the calling warp, each lane's column of the next
+// rows copied ahead into the warp's staging slots sUw. Zones that need the FP64 recovery go to
 // the stage's list (a.high).
 template <int DT>
 __device__ __forceinline__ void recover_rows_tile(const StageArgs& a, const int4 t, double (*sUw)[NFIELD][32],
-                                                  MlpWeights& W, C2pStats& st) {
+                                                  MlpWeights& W, C2pStats& st, int most = TILE_R) {
     const int lane = threadIdx.x & 31;
     const DevBlock& B = a.blocks[t.x];
     const int j = t.z + lane;
     const bool jin = j < B.nq;
-    const int rows = min(TILE_R, B.nr - t.y);
+    const int rows = min(most, B.nr - t.y);
     const int64_t n = (int64_t)B.nr * B.nq;
     const double* Ub = B.buf[a.sel_in] + (int64_t)t.y * B.nq + j;
     auto issue = [&](int r) {
@@ -442,8 +442,12 @@ __global__ void __launch_bounds__(TILE_THREADS, 3) c2p_rows_kernel(StageArgs a) 
     MlpWeights& W = *reinterpret_cast<MlpWeights*>(smem_raw);   // unused without the learned guess
     const int w = threadIdx.x >> 5;
     C2pStats st;
-    for (int tile = blockIdx.x * WPC + w; tile < a.ntiles; tile += gridDim.x * WPC)
-        recover_rows_tile<DT>(a, a.tiles[tile], sU[w], W, st);
+    const int split = a.row_split, part_rows = TILE_R / split;
+    for (int item = blockIdx.x * WPC + w; item < a.ntiles * split; item += gridDim.x * WPC) {
+        int4 t = a.tiles[item / split];
+        t.y += (item % split) * part_rows;
+        if (t.y < a.blocks[t.x].nr) recover_rows_tile<DT>(a, t, sU[w], W, st, part_rows);
+    }
     cp_async_wait<0>();
     warp_reduce_stats(a.status, st.zones, st.it64, st.it32, st.fbs, st.dtz, a.compute_dt != 0);
 }
@@ -532,11 +536,16 @@ cudaError_t launch_c2p_mixed(const StageArgs& a, cudaStream_t s) {
     if (a.ntiles <= 0) return cudaSuccess;
     if (a.high) {
         // every zone in FP32; the ones that need the FP64 recovery, densely after
-        // one warp per recovery tile
-        const int wt = (a.ntiles + TILE_THREADS / 32 - 1) / (TILE_THREADS / 32);
+        // one warp per recovery tile; on a small grid, whose tiles would not
+        // give every SM partition two warps, 2, 4 or 8 of them (259 x 93 zones:
+        // 15.6 us with one, 7.3 with 8)
+        StageArgs y = a;
+        y.row_split = 1;
+        while (y.row_split < TILE_R && a.ntiles * y.row_split < 8 * num_sms()) y.row_split *= 2;
+        const int wt = (a.ntiles * y.row_split + TILE_THREADS / 32 - 1) / (TILE_THREADS / 32);
         auto k = a.compute_dt ? c2p_rows_kernel<1> : c2p_rows_kernel<0>;
         const int grid = std::min(wt, resident_grid(k, TILE_THREADS, 0));
-        cudaError_t e = launch_chained(k, grid, TILE_THREADS, 0, s, a);
+        cudaError_t e = launch_chained(k, grid, TILE_THREADS, 0, s, y);
         if (e != cudaSuccess) return e;
         if (a.mlp) {
             const size_t bytes = sizeof(MlpWeights) + 8 * MLP_ACT_ELEMS * sizeof(__nv_bfloat16);

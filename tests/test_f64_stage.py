@@ -98,3 +98,23 @@ def test_host_state_chunks_on_a_larger_grid(precision, order):
     s.get_state(want_c, want_s)
     assert np.array_equal(co.array, want_c) and np.array_equal(so.array, want_s)
     assert not np.array_equal(co.array, ci.array)
+
+
+@pytest.mark.parametrize("nr,nq,zones", [(5, 40, 90), (13, 97, 210), (40, 333, 330), (64, 700, 500)])
+def test_small_mixed_grids_split_strips_and_tiles(nr, nq, zones):
+    """Grids that give a warp less than a whole strip or recovery tile (8, 4, 2
+    and 1 warps per tile): the bits of the tile form."""
+    import knc
+    from knc import workloads
+    w = workloads.jet_small()
+    w.mesh.block_size = nr
+    w.mesh.num_radial_zones = zones
+    w.mesh.num_polar_zones = nq
+    states = []
+    for t in (dict(tile_rows=8), dict(tile_rows=16, strip=True, deferred=True)):
+        g = knc.build_solver(w)
+        g.set_precision(knc.abi.KNC_PRECISION_MIXED)
+        g.set_tuning(**t)
+        g.advance(4)
+        states.append(g.state())
+    assert max(zone_relative_errors(states[1], states[0])) == 0.0
