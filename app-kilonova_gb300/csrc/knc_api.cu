@@ -231,9 +231,6 @@ void free_block(BlockH& b) {
 // 1.358, 1.379 ms).
 constexpr int STREAM_STRIP_ROWS = 4;
 
-// Strips per SM partition that a small grid's mixed update is spread to.
-constexpr int64_t MIXED_STRIPS = 2;
-
 // The FP64 update's items {slot, i0, j0, rows} (32 columns each,
 // knc_f64_update.cu) of the blocks slot0, slot0 + 1, ... with the given (nr,
 // nq), where the caller has not chosen their rows. An item costs about one
@@ -280,6 +277,39 @@ std::vector<int4> f64_items(const std::vector<std::pair<int64_t, int64_t>>& shap
     return items;
 }
 
+// The mixed update's warp strips {slot, i0, j0, rows} of the blocks 0, 1, ...
+// (separate stage), `most` rows high at most (the caller's tile_rows), their
+// offsets per block in `off`. The SMs take CTAs of 4 strips in list order, so
+// the same rule as f64_items fills the last round: 16-row strips throughout
+// on one resident grid left a warp with 3 or 4 of them (4096 x 1024: 9472
+// strips on 3040 warps). Fold of the 4096 x 1024 wind 12.05 -> 11.7 ms,
+// 2048 x 512 jet 4.34 -> 4.19 ms (over 2, 3, 6, 10: 4.49, 4.25, 4.15, 4.51),
+// uneven blocks 2.61 -> 2.56 ms; seven 37 x 93 blocks, ten steps, 1.57 ms ->
+// 1.26 (least 1, 2, 6, 8 rows: 1.39, 1.46, 1.26, 1.32).
+constexpr double MIXED_ROWS_OVER = 4.0, MIXED_ROWS_LEAST = 4.0;
+
+std::vector<int4> mixed_strips(const std::vector<std::pair<int64_t, int64_t>>& shapes, int sms, int64_t most,
+                               std::vector<int>& off) {
+    auto columns = [](int64_t nq) { return (nq + STRIP_OUT - 1) / STRIP_OUT; };
+    double left = 0.0;   // rows of STRIP_OUT columns left, per SM partition
+    for (const auto& s : shapes) left += (double)(s.first * columns(s.second)) / (4.0 * sms);
+    std::vector<int4> strips;
+    off.clear();
+    for (size_t k = 0; k < shapes.size(); ++k) {
+        const int64_t nr = shapes[k].first, nq = shapes[k].second;
+        off.push_back((int)strips.size());
+        for (int64_t i0 = 0; i0 < nr;) {
+            const int64_t want = std::min<int64_t>((int64_t)std::max(left / MIXED_ROWS_OVER, MIXED_ROWS_LEAST), most);
+            const int64_t per = (nr - i0 + want - 1) / want, rows = (nr - i0 + per - 1) / per;
+            for (int64_t j0 = 0; j0 < nq; j0 += STRIP_OUT)
+                strips.push_back(make_int4((int)k, (int)i0, (int)j0, (int)rows));
+            i0 += rows;
+            left -= (double)(rows * columns(nq)) / (4.0 * sms);
+        }
+    }
+    return strips;
+}
+
 // One block set's device view.
 struct Layout {
     DevBlock* d_table = nullptr;
@@ -293,7 +323,7 @@ struct Layout {
     int utr = 0;
     int uform = -1;
     int list_cols = 0;          // columns of a strip: 32 for the FP64 update's items, else STRIP_OUT
-    bool list_auto = false;     // item rows by f64_items
+    bool list_auto = false;     // item or strip rows by f64_items or mixed_strips
     bool f64_tiles = false;     // the utiles are tiles of TILE64_COLS columns
     int64_t nzones = 0;         // zones of the block set
     TmaMaps* d_tmaps = nullptr; // tensor maps per slot (tiles of `utr` rows), when every block allows them
@@ -688,21 +718,13 @@ int rebuild_table(knc_ctx* c) {
     const bool rows64 = c->precision != KNC_PRECISION_MIXED && !c->fused;
     const bool rows_auto = rows64 && !c->utr_set;
     const int cols = rows64 ? TILE_Q : STRIP_OUT;
+    const bool guided = c->uform == KNC_UPDATE_STRIP && !rows64 && !c->fused;   // strips by mixed_strips
     if (!c->dirty && L(c).utr == c->utr && L(c).uform == c->uform && L(c).chunk_nt == fused_threads(c) &&
-        L(c).list_cols == cols && L(c).list_auto == rows_auto)
+        L(c).list_cols == cols && L(c).list_auto == (rows_auto || guided))
         return KNC_OK;
     const int64_t item_rows = rows64 ? std::min<int64_t>(c->utr, 32) : c->utr;
-    // Warp strips are utr rows high at most: where that would leave the mixed
-    // stage fewer than MIXED_STRIPS strips per SM partition, lower ones (a strip
-    // is a latency chain along its rows).
-    int64_t strip_rows = item_rows;
-    if (!rows64 && !c->fused) {
-        int64_t total = 0;
-        for (auto& kv : c->blocks) total += kv.second.nr * ((kv.second.nq + cols - 1) / cols);
-        strip_rows = std::min(strip_rows, std::max<int64_t>(1, total / (MIXED_STRIPS * 4 * c->sms)));
-    }
     L(c).list_cols = cols;
-    L(c).list_auto = rows_auto;
+    L(c).list_auto = rows_auto || guided;
     const int nb = (int)c->blocks.size();
     std::vector<DevBlock> tab(nb);
     std::vector<int4> tiles, utiles, chunks, strips;
@@ -782,17 +804,17 @@ int rebuild_table(knc_ctx* c) {
         for (int64_t i0 = 0; i0 < b.nr; i0 += TILE_R)
             for (int64_t j0 = 0; j0 < b.nq; j0 += TILE_Q)
                 tiles.push_back(make_int4(slot, (int)i0, (int)j0, (int)zoff));
-        if (c->uform == KNC_UPDATE_STRIP) {
+        if (c->uform == KNC_UPDATE_STRIP && !guided) {
             // ceil(nr / utr) strips per column, their heights as even as
             // whole rows allow (64 rows at utr 13: 13, 13, 13, 13, 12)
-            const int64_t per = (b.nr + strip_rows - 1) / strip_rows;
+            const int64_t per = (b.nr + item_rows - 1) / item_rows;
             for (int64_t j0 = 0; j0 < b.nq; j0 += cols)
                 for (int64_t k = 0, i0 = 0; k < per; ++k) {
                     const int64_t rows = b.nr / per + (k < b.nr % per ? 1 : 0);
                     strips.push_back(make_int4(slot, (int)i0, (int)j0, (int)rows));
                     i0 += rows;
                 }
-        } else if (!rows_auto) {
+        } else if (c->uform != KNC_UPDATE_STRIP && !rows_auto) {
             for (int64_t i0 = 0; i0 < b.nr; i0 += item_rows)
                 for (int64_t j0 = 0; j0 < b.nq; j0 += TILE_Q)
                     utiles.push_back(make_int4(slot, (int)i0, (int)j0, (int)std::min<int64_t>(item_rows, b.nr - i0)));
@@ -805,9 +827,10 @@ int rebuild_table(knc_ctx* c) {
         prev = &b;
         ++slot;
     }
+    std::vector<std::pair<int64_t, int64_t>> shapes;
+    for (const BlockH* b : order) shapes.push_back({b->nr, b->nq});
+    if (guided) strips = mixed_strips(shapes, c->sms, c->utr, L(c).strip_off);
     if (rows_auto) {
-        std::vector<std::pair<int64_t, int64_t>> shapes;
-        for (const BlockH* b : order) shapes.push_back({b->nr, b->nq});
         utiles = f64_items(shapes, 0, c->sms, L(c).f64_tiles);
     } else {
         L(c).f64_tiles = false;

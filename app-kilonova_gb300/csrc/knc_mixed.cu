@@ -671,8 +671,8 @@ template <int MB>
 static void update_strips(const StageArgs& a, cudaStream_t s) {
     // (with a list at least one CTA per SM: its zones are claimed by every warp)
     const int want = std::max((a.nstrips + STRIP_WARPS - 1) / STRIP_WARPS, a.hp_list ? num_sms() : 1);
-    const int grid = std::min(want, resident_grid(update_strip_kernel<float, true, MB>, STRIP_WARPS * 32, 0));
-    launch_chained(update_strip_kernel<float, true, MB>, grid, STRIP_WARPS * 32, 0, s, a);
+    // a CTA of warps per STRIP_WARPS strips, taken by the SMs as they come free
+    launch_chained(update_strip_kernel<float, true, MB>, want, STRIP_WARPS * 32, 0, s, a);
 }
 
 cudaError_t launch_update_mixed(const StageArgs& a, cudaStream_t s) {
