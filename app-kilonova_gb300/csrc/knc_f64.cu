@@ -111,7 +111,7 @@ __global__ void __launch_bounds__(TILE_THREADS, MLP ? 1 : 4) c2p_f64_kernel(Stag
         const int j = t.z + threadIdx.x % TILE_Q;
         F64C2p<MLP>::zone(a, t.x, B, i, j, i < B.nr && j < B.nq, W, act, st);
     }
-    warp_reduce_stats(a.status, st.zones, st.it64, 0ull, st.fbs, st.dtz, a.compute_dt != 0);
+    cta_reduce_stats<TILE_THREADS / 32>(a.status, st.zones, st.it64, 0ull, st.fbs, st.dtz, a.compute_dt != 0);
 }
 
 // ---- the fused stage (FP64) ----------------------------------------------------
