@@ -31,6 +31,7 @@ constexpr int TILE_THREADS = TILE_R * TILE_Q;
 constexpr int NFIELD = 5;
 constexpr int STRIP_OUT = TILE_Q - 4;   // output columns of a warp strip (2 halo lanes each side)
 constexpr int STRIP_WARPS = 4;          // independent strips per CTA
+constexpr int C2P_ROWS_CTAS = 3;        // resident CTAs per SM of the row-walking recovery (TILE_THREADS threads)
 constexpr int TILE64_COLS = 31;         // columns of an FP64 update tile: their 32 polar faces fill a warp
 
 struct DevBlock {
@@ -172,7 +173,12 @@ struct StageArgs {
     unsigned* high_count;       // this stage's count (status word, by stage parity)
     unsigned* high_count_next;  // the next stage's, cleared by the dense pass
     unsigned high_cap;          // entries a.high holds
-    int32_t row_split;          // row-walking recovery: warps per recovery tile (1, 2, 4 or 8)
+    // row-walking recovery: the runs {slot, i0, j0, rows} of 32 columns that warp
+    // k walks are runs[run_off[k]] .. runs[run_off[k + 1] - 1], for run_warps
+    // warps (a multiple of a CTA's)
+    const int4* runs;
+    const int* run_off;
+    int32_t run_warps;
     int32_t avg_half;       // w1 == bf == 1/2 (the RK2 average, halved exactly on the integer pipe)
     const float* mlp;       // packed MLP weights (device) or null
     DevStatus* status;

@@ -371,12 +371,12 @@ __global__ void __launch_bounds__(TILE_THREADS, 3) c2p_mixed_kernel(StageArgs a)
     warp_reduce_stats(a.status, st.zones, st.it64, st.it32, st.fbs, st.dtz, a.compute_dt != 0);
 }
 
-// ---- recovery by warps walking the rows of a tile -----------------------------
+// ---- recovery by warps walking rows --------------------------------------------
 // The recovery's arithmetic between its loads and its stores is long and
 // serial, so a zone-per-thread loop keeps few loads in flight and runs
-// latency-bound. Here a warp takes a whole recovery tile (TILE_R rows of 32
-// zones): the tile's descriptor and block fields are read once instead of once
-// per zone, and each lane copies its column's state of the rows C2P_DEPTH - 1
+// latency-bound. Here a warp takes a run of rows of 32 zones (a.runs; the
+// fused stage's warps whole recovery tiles): its descriptor and block fields
+// are read once instead of once per zone, and each lane copies its column's state of the rows C2P_DEPTH - 1
 // ahead into shared memory with cp.async (8-byte, L1-allocating) while it
 // recovers the current row, so the copies hold no registers. A lane reads
 // only the slots it filled (no barrier); cp.async.wait_group orders its own
@@ -397,8 +397,8 @@ __device__ __forceinline__ void cp_async_wait() {
 
 // Rows i0 .. i0 + most - 1 (as far as the block goes) of a recovery tile t =
 // {slot, i0, j0, -} walked by the calling warp, each lane's column of the next
-// rows copied ahead into the warp's staging slots sUw. Zones that need the FP64 recovery go to
-// the stage's list (a.high).
+// rows copied ahead into the warp's staging slots sUw. Zones that need the
+// FP64 recovery go to the stage's list (a.high).
 template <int DT>
 __device__ __forceinline__ void recover_rows_tile(const StageArgs& a, const int4 t, double (*sUw)[NFIELD][32],
                                                   MlpWeights& W, C2pStats& st, int most = TILE_R) {
@@ -431,7 +431,7 @@ __device__ __forceinline__ void recover_rows_tile(const StageArgs& a, const int4
 }
 
 template <int DT>
-__global__ void __launch_bounds__(TILE_THREADS, 3) c2p_rows_kernel(StageArgs a) {
+__global__ void __launch_bounds__(TILE_THREADS, C2P_ROWS_CTAS) c2p_rows_kernel(StageArgs a) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     constexpr int WPC = TILE_THREADS / 32;
     __shared__ __align__(16) double sU[WPC][C2P_DEPTH][NFIELD][32];
@@ -442,11 +442,10 @@ __global__ void __launch_bounds__(TILE_THREADS, 3) c2p_rows_kernel(StageArgs a) 
     MlpWeights& W = *reinterpret_cast<MlpWeights*>(smem_raw);   // unused without the learned guess
     const int w = threadIdx.x >> 5;
     C2pStats st;
-    const int split = a.row_split, part_rows = TILE_R / split;
-    for (int item = blockIdx.x * WPC + w; item < a.ntiles * split; item += gridDim.x * WPC) {
-        int4 t = a.tiles[item / split];
-        t.y += (item % split) * part_rows;
-        if (t.y < a.blocks[t.x].nr) recover_rows_tile<DT>(a, t, sU[w], W, st, part_rows);
+    const int wk = blockIdx.x * WPC + w;
+    for (int k = a.run_off[wk]; k < a.run_off[wk + 1]; ++k) {
+        const int4 t = a.runs[k];
+        recover_rows_tile<DT>(a, t, sU[w], W, st, t.w);
     }
     cp_async_wait<0>();
     warp_reduce_stats(a.status, st.zones, st.it64, st.it32, st.fbs, st.dtz, a.compute_dt != 0);
@@ -536,16 +535,9 @@ cudaError_t launch_c2p_mixed(const StageArgs& a, cudaStream_t s) {
     if (a.ntiles <= 0) return cudaSuccess;
     if (a.high) {
         // every zone in FP32; the ones that need the FP64 recovery, densely after
-        // one warp per recovery tile; on a small grid, whose tiles would not
-        // give every SM partition two warps, 2, 4 or 8 of them (259 x 93 zones:
-        // 15.6 us with one, 7.3 with 8)
-        StageArgs y = a;
-        y.row_split = 1;
-        while (y.row_split < TILE_R && a.ntiles * y.row_split < 8 * num_sms()) y.row_split *= 2;
-        const int wt = (a.ntiles * y.row_split + TILE_THREADS / 32 - 1) / (TILE_THREADS / 32);
+        // one resident grid, a warp per entry of a.run_off
         auto k = a.compute_dt ? c2p_rows_kernel<1> : c2p_rows_kernel<0>;
-        const int grid = std::min(wt, resident_grid(k, TILE_THREADS, 0));
-        cudaError_t e = launch_chained(k, grid, TILE_THREADS, 0, s, y);
+        cudaError_t e = launch_chained(k, a.run_warps / (TILE_THREADS / 32), TILE_THREADS, 0, s, a);
         if (e != cudaSuccess) return e;
         if (a.mlp) {
             const size_t bytes = sizeof(MlpWeights) + 8 * MLP_ACT_ELEMS * sizeof(__nv_bfloat16);

@@ -100,10 +100,11 @@ def test_host_state_chunks_on_a_larger_grid(precision, order):
     assert not np.array_equal(co.array, ci.array)
 
 
-@pytest.mark.parametrize("nr,nq,zones", [(5, 40, 90), (13, 97, 210), (40, 333, 330), (64, 700, 500)])
-def test_small_mixed_grids_split_strips_and_tiles(nr, nq, zones):
-    """Grids that give a warp less than a whole strip or recovery tile (8, 4, 2
-    and 1 warps per tile): the bits of the tile form."""
+@pytest.mark.parametrize("nr,nq,zones", [(5, 40, 90), (13, 97, 210), (40, 240, 330), (64, 700, 500)])
+def test_mixed_strips_and_recovery_runs(nr, nq, zones):
+    """Strips and recovery runs of one to many rows, with and without columns
+    that fill a CTA (97 and 700 zones: 4 and 22 columns of 32; 240: 8): the bits
+    of the tile form."""
     import knc
     from knc import workloads
     w = workloads.jet_small()
