@@ -263,8 +263,10 @@ int knc_set_batched(knc_ctx* ctx, int32_t graph);
 /* Launch shape of a stage (no counterpart in the reference, whose stage is a
  * Rayon/Tokio task per block, src/scheme.rs:16-173).
  *   tile_rows    radial rows of an update tile (4, 8 or 16; 32 polar columns;
- *                a tile runs on (tile_rows + 1) warps), or of a warp strip
- *                (4 to 64)
+ *                a tile runs on (tile_rows + 1) warps), or at most of a warp
+ *                strip (4 to 64; lower towards the end of the grid). In the
+ *                separate FP64 stage: rows of a warp's item of 32 columns (32
+ *                at most; chosen by the grid while no tuning is set)
  *   fused        0: a stage is four launches (ghost rows, recovery, remaps,
  *                update; the deferring recovery adds its dense pass); 1: one
  *                persistent cooperative launch whose phases are separated by
