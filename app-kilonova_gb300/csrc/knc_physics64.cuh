@@ -54,26 +54,33 @@ __device__ __forceinline__ float estimate_f32(double x) {
 // moves right (left), 0: undecided. The FP32 estimate of a^2 and b^2, whose
 // difference decides the sign of the wave speed (a -+ b) / (1 - v^2 cs^2), is
 // good to 1e-4 for k = 1 - cs^2 > 0.01; the FP64 expression it stands for
-// itself to 1e-8 for W^2 < 1e8; the margin is 2%. False for NaNs.
+// itself to 1e-8 for W^2 < 1e8; the margin is 2%. That holds for numbers the
+// estimate neither saturates nor flushes: rho and p (unless it is zero) inside
+// FP32's normal range with room for p / rho, and u_n^2 far above the smallest
+// FP32 number, so that what underflows on the way to b^2 is too small to
+// matter against a^2. Everything else is undecided, NaNs among it (they
+// saturate, above every upper bound here).
 template <bool SRHD>
 __device__ __forceinline__ int sure_direction(float gm, float gh, const double* P, int axis) {
     const float rho = estimate_f32(P[0]), pre = estimate_f32(P[3]);
     const float un = estimate_f32(axis == 0 ? P[1] : P[2]);
-    const float t = pre / rho;
+    const float t = pre / rho, u2 = un * un;
     bool sure;
     if (SRHD) {
         const float ut = estimate_f32(axis == 0 ? P[2] : P[1]);
-        const float w2 = 1.0f + un * un + ut * ut;
+        const float w2 = 1.0f + u2 + ut * ut;
         const float o = 1.0f / w2;                     // 1 - v^2
         const float c2 = gm * t / (1.0f + gh * t);
         const float k = 1.0f - c2;
-        const float a2 = un * un * o * k * k;
+        const float a2 = u2 * o * k * k;
         const float b2 = c2 * o * (o + ut * ut * o * k);
         sure = w2 < 1e8f && k > 0.01f && a2 > 1.02f * b2;
     } else {
-        sure = un * un > 1.02f * gm * t && un * un < 1e30f;
+        sure = u2 > 1.02f * gm * t;
     }
-    sure = sure && rho > 1e-30f && rho < 1e30f && t >= 0.0f && t < 1e30f;
+    const bool cold = ((hi_word(P[3]) << 1) | lo_word(P[3])) == 0u;
+    sure = sure && rho > 1e-30f && rho < 1e30f && (cold || (pre > 1e-36f && pre < 1e36f)) && t < 1e30f &&
+           u2 > 1e-30f && u2 < 1e30f;
     return sure ? (un > 0.0f ? 1 : -1) : 0;
 }
 
