@@ -79,7 +79,10 @@ __device__ __forceinline__ Start64 start_sum(uint32_t R, int32_t c, float r) {
 // mantissa as a fraction of 2^63; R 2^-24 the FP32 estimate of 1 / m, in
 // [0.5, 1); the residual e = 1 - m R 2^-24 (below 1.5 2^-23) in units of 2^-53
 // from the exact product's low words (its leading bits cancel); then
-// 1 / m = R 2^-24 (1 + e + e^2).
+// 1 / m = R 2^-24 (1 + e + e^2). The estimate of a 24-bit number between 2^31
+// and 2^32 is never below 2^-32, as R's bits assume (its 2^23 operands, and
+// the 2^24 of the root's, are swept by tests/test_fp64_starts.py); a lower
+// clamp beside the upper one cost 0.3% of the FP64 step.
 __device__ __forceinline__ Start64 rcp_start(double b) {
     const uint32_t hi = hi_word(b), lo = lo_word(b);
     const uint32_t Mh = __funnelshift_l(lo, hi, 11) | 0x80000000u, Ml = lo << 11;
@@ -114,9 +117,11 @@ __device__ __forceinline__ Start64 rsqrt_start(double x) {
     return start_sum(R, __float2int_rn(r0 * (t * 9007199254740992.0f)), r0);
 }
 
-// k = R / D rounded to the nearest integer, f its FP32 value (|k| < 2^12, f to
-// 2^-13): the quotient Q + k is the correctly rounded one unless f lies next to
-// a midpoint, which `near` says.
+// k = R / D rounded to the nearest integer, f its FP32 value: the quotient
+// Q + k is the correctly rounded one unless f lies next to a midpoint, which
+// `near` says. |k| is a few units after rcp_start and up to 2^9 after
+// rsqrt_start (2^-44 of 2^53), and stays below 2^10 (a remainder's upper word
+// is an int32); f is good to 2^-22 |k| + 2^-20 < 2^-11, the guard below.
 __device__ __forceinline__ int nearest(float f, bool& near) {
     const float kf = rintf(f);
     near = fabsf(f - kf) > 0.4995f;
