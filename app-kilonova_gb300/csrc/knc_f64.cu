@@ -94,8 +94,7 @@ struct F64C2p {
 template <bool MLP>
 __global__ void __launch_bounds__(TILE_THREADS, MLP ? 1 : 4) c2p_f64_kernel(StageArgs a) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
-    const unsigned long long ek = *(volatile unsigned long long*)&a.status->err_key;
-    if (ek != NO_ERROR && (uint32_t)(ek >> 48) < (uint32_t)a.stage) return;
+    if (cta_any(stopped_before(a))) return;
     MlpWeights& W = *reinterpret_cast<MlpWeights*>(smem_raw);
     __nv_bfloat16* act = reinterpret_cast<__nv_bfloat16*>(smem_raw + sizeof(MlpWeights)) +
                          (threadIdx.x >> 5) * MLP_ACT_ELEMS;

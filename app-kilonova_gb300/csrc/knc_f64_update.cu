@@ -291,7 +291,7 @@ __global__ void __launch_bounds__(ROWS64_WARPS * 32, 3)
     __shared__ Edge64 sE[ROWS64_WARPS];
     // A failed c2p in this or an earlier stage stops the step: keep the
     // input state untouched so the failure can be reported from it.
-    if (*(volatile unsigned long long*)&a.status->err_key != NO_ERROR) return;
+    if (stopped(a)) return;   // (the same for a warp's lanes, and its warps are on their own)
     const PhysT<double> ph = make_phys<double>(a);
     const int w = threadIdx.x >> 5;
     for (int k = blockIdx.x * ROWS64_WARPS + w; k < nitems; k += gridDim.x * ROWS64_WARPS)
@@ -319,7 +319,7 @@ template <bool SRHD, bool HLLC>
 __global__ void __launch_bounds__(ROWS64_WARPS * 32, 3)
     update_tile64_kernel(const __grid_constant__ StageArgs a, const int4* __restrict__ items) {
     __shared__ Tile64 T;
-    if (*(volatile unsigned long long*)&a.status->err_key != NO_ERROR) return;
+    if (cta_any(stopped(a))) return;
     const PhysT<double> ph = make_phys<double>(a);
     const int4 it = items[blockIdx.x];
     const DevBlock& B = a.blocks[it.x];

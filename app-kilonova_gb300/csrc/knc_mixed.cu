@@ -351,8 +351,8 @@ struct MixedC2p {
 template <bool MLP>
 __global__ void __launch_bounds__(TILE_THREADS, 3) c2p_mixed_kernel(StageArgs a) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
-    const unsigned long long ek = *(volatile unsigned long long*)&a.status->err_key;
-    if (ek != NO_ERROR && (uint32_t)(ek >> 48) < (uint32_t)a.stage) return;
+    const bool stop = stopped_before(a);
+    if (MLP ? cta_any(stop) : stop) return;   // (the warps meet where they load the weights)
     MlpWeights& W = *reinterpret_cast<MlpWeights*>(smem_raw);
     __nv_bfloat16* act = reinterpret_cast<__nv_bfloat16*>(smem_raw + sizeof(MlpWeights)) +
                          (threadIdx.x >> 5) * MLP_ACT_ELEMS;
