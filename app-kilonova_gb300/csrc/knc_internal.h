@@ -265,6 +265,7 @@ cudaError_t launch_c2p_f64(const StageArgs& a, cudaStream_t s);
 // a.utiles), 32 columns each, or tiles of at most 2 rows x TILE64_COLS columns
 // (a.f64_tiles) (knc_f64_update.cu).
 cudaError_t launch_update_f64(const StageArgs& a, cudaStream_t s);
+cudaError_t launch_f32_forms(const float* in, int64_t n, float* out);   // n pairs, 8 n results (knc_test_f32_forms)
 cudaError_t launch_ghost_f64(const GhostArgs& a, cudaStream_t s);
 cudaError_t launch_ghost_mixed(const GhostArgs& a, cudaStream_t s);
 cudaError_t launch_c2p_mixed(const StageArgs& a, cudaStream_t s);

@@ -531,6 +531,28 @@ static int resident_grid(K kernel, int threads, size_t smem) {
     return cache[key] = per_sm * num_sms();
 }
 
+// The one-instruction forms beside the plain ones, as this unit compiles them
+// (knc_test_f32_forms).
+__global__ void f32_forms_kernel(const float* in, int64_t n, float* out) {
+    const int64_t k = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (k >= n) return;
+    const float a = in[2 * k], b = in[2 * k + 1];
+    float* o = out + 8 * k;
+    o[0] = rcp_n(b);
+    o[1] = 1.0f / b;
+    o[2] = sqrt_n(b);
+    o[3] = sqrtf(b);
+    o[4] = rsqrt_n(b);
+    o[5] = rsqrtf(b);
+    o[6] = a * rcp_n(b);
+    o[7] = a / b;
+}
+
+cudaError_t launch_f32_forms(const float* in, int64_t n, float* out) {
+    f32_forms_kernel<<<(unsigned)((n + 255) / 256), 256>>>(in, n, out);
+    return cudaGetLastError();
+}
+
 cudaError_t launch_c2p_mixed(const StageArgs& a, cudaStream_t s) {
     if (a.ntiles <= 0) return cudaSuccess;
     if (a.high) {

@@ -291,12 +291,17 @@ __device__ __forceinline__ void riemann(const PhysT<R>& ph, const R* pl, const R
 }
 
 // ---- FP32 relativistic forms for the mixed stage ------------------------------
-// Reciprocals and roots of numbers that are never subnormal (Lorentz factors,
-// enthalpies, 1 - v^2 cs^2, wave-speed differences, volumes in the stage's
-// length unit): one hardware instruction, without the scaling that the plain
-// forms put around it for subnormal operands. On normal numbers they give the
-// bits of 1.0f / x, sqrtf(x) and rsqrtf(x) as this unit compiles them, and
-// a * rcp_n(b) those of a / b (checked over every mantissa).
+// Reciprocals and roots in one hardware instruction, without the scaling that
+// the plain forms put around it for subnormal numbers: operands below 2^-126
+// count as zero, and so does 1 / x for x above 2^126. Everywhere else they give
+// the bits of 1.0f / x, sqrtf(x) and rsqrtf(x) as the mixed stage's unit
+// compiles them, and a * rcp_n(b) those of a / b (tests/test_f32_forms.py sweeps
+// every mantissa). The operands: Lorentz factors, enthalpies, 1 + tau / D + p / D
+// (at least 1), 1 - v^2 and 1 - v^2 cs^2, radii and volumes in the stage's
+// length unit, and three that can be subnormal: |S|^2 / D^2 (compared with a
+// number near 1), the radicand of the sound's part of a wave speed (a part below
+// 1.1e-19 of the speed of light vanishes, 12 digits below what an FP32 flux
+// resolves), and the difference of the outer wave speeds (hlle_f32x2 bounds it).
 __device__ __forceinline__ float rcp_n(float x) {
     float r;
     asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
@@ -397,7 +402,9 @@ __device__ __forceinline__ void hlle_f32x2(const Side<float>& L, const Side<floa
         for (int q = 0; q < 4; ++q) out[q] = R.F[q];
         out[4] = R.sF;
     } else {
-        const float inv = rcp_n(ap - am);
+        // (a subnormal difference, am < 0 < ap in gas without pressure, would
+        // give an infinite reciprocal and 0 x infinity below)
+        const float inv = rcp_n(fmaxf(ap - am, 1.17549435e-38f));
         const float apam = ap * am;
         const float2 AP = bcast(ap), MAM = bcast(-am), APAM = bcast(apam), INV = bcast(inv);
 #pragma unroll

@@ -11,6 +11,7 @@
 #include "../../include/knc.h"
 #include "knc_bits.cuh"
 #include "knc_fp64.cuh"
+#include "knc_internal.h"
 
 namespace {
 
@@ -72,6 +73,22 @@ extern "C" int knc_test_fp64_ops(const double* in, int64_t n, double* out) {
         e = cudaGetLastError();
     }
     if (e == cudaSuccess) e = cudaMemcpy(out, d_out, n * 48, cudaMemcpyDeviceToHost);
+    cudaFree(d_in);
+    cudaFree(d_out);
+    return e == cudaSuccess ? KNC_OK : KNC_ERR_CUDA;
+}
+
+extern "C" int knc_test_f32_forms(const float* in, int64_t n, float* out) {
+    if (!in || !out || n <= 0) return KNC_ERR_INVALID_ARGUMENT;
+    float *d_in = nullptr, *d_out = nullptr;
+    if (cudaMalloc(&d_in, n * 8) != cudaSuccess) return KNC_ERR_OUT_OF_MEMORY;
+    if (cudaMalloc(&d_out, n * 32) != cudaSuccess) {
+        cudaFree(d_in);
+        return KNC_ERR_OUT_OF_MEMORY;
+    }
+    cudaError_t e = cudaMemcpy(d_in, in, n * 8, cudaMemcpyHostToDevice);
+    if (e == cudaSuccess) e = knc::launch_f32_forms(d_in, n, d_out);
+    if (e == cudaSuccess) e = cudaMemcpy(out, d_out, n * 32, cudaMemcpyDeviceToHost);
     cudaFree(d_in);
     cudaFree(d_out);
     return e == cudaSuccess ? KNC_OK : KNC_ERR_CUDA;

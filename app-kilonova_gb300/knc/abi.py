@@ -216,6 +216,7 @@ SIGNATURES = {
     "knc_measure_fp64_peak": (C.c_int, [_DP]),
     "knc_test_conversions": (C.c_int, [_DP, C.c_int64, _DP]),
     "knc_test_fp64_ops": (C.c_int, [_DP, C.c_int64, _DP]),
+    "knc_test_f32_forms": (C.c_int, [_FP, C.c_int64, _FP]),
     "knc_recover_primitives_noalloc": (C.c_int, [C.POINTER(HydroParams), C.POINTER(MeshParams), C.c_int32,
                                                  _P, _P, _P, _P, C.POINTER(Error)]),
 }

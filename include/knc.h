@@ -479,6 +479,11 @@ int knc_test_conversions(const double* in, int64_t n, double* out);
  * out[6 * k + 0..5] = (a / b, 1 / b, sqrt|b|, a / sqrt|b|, min(a, b), max(a, b)). */
 int knc_test_fp64_ops(const double* in, int64_t n, double* out);
 
+/* Self-test of the mixed stage's one-instruction reciprocal, square root and
+ * reciprocal root: for n pairs (a, b) = in[2 * k + 0..1] writes out[8 * k + 0..7]
+ * = each form beside the plain one: of 1 / b, sqrt(b), 1 / sqrt(b), a / b. */
+int knc_test_f32_forms(const float* in, int64_t n, float* out);
+
 /* Measured FP64 FMA throughput of the current device (GFLOP/s, 2/FMA). */
 int knc_measure_fp64_peak(double* gflops);
 
