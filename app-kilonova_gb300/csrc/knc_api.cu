@@ -240,19 +240,31 @@ constexpr int STREAM_STRIP_ROWS = 4;
 // work left (guided self-scheduling, Polychronopoulos and Kuck 1987): the rows
 // left per SM partition over 1.5, at most 16, at least 2. 2048 x 512 jet fold
 // 5.22 (8 rows throughout) -> 4.78 ms, over 1, 2, 3: 4.74, 4.94, 5.00;
-// Newtonian sphere 4.12 -> 3.83 ms. Grids under 16 rows per partition take 2
-// throughout (450 x 230, RK3: 2 rows 1.10 ms, 3 to 4 1.18, 1 1.36; 256 x 128:
-// 2 rows 235 us, 1 229, 3 267). Grids under 8 rows per partition take tiles
-// instead (`tiles`): rows per partition, items and tiles in us: 0.4 (Newtonian
-// sphere) 283, 213; 5.9 (RK3 HLLC) 995, 942; 10 (wind) 1037, 1009, (sphere)
-// 984, 986; 20 (sphere) 1650, 1743.
-constexpr double F64_ROWS_OVER = 1.5, F64_ROWS_LEAST = 2.0, F64_ROWS_MOST = 16.0, F64_ROWS_SMALL_GRID = 16.0;
+// Newtonian sphere 4.12 -> 3.83 ms. Grids of 12 to 24 rows per partition take
+// 8 throughout, three items or fewer to a partition, which holds three warps:
+// one wave (wind, sphere of 512 columns in us, 2 rows or by the work left -> 8:
+// 12.6 rows 575 -> 472, 531 -> 417; 16 660 -> 498, 598 -> 423; 20 744 -> 675, 673
+// -> 597; 23.6 841 -> 695, 761 -> 610; above 24 a second wave: 26 1001 -> 1024, 906
+// -> 935), smaller ones 2 (8 against 2 rows: 8.4 rows 436 -> 456, 407 -> 417;
+// 11.8 463 -> 461, 419 -> 417). Grids under 8 rows per partition take tiles
+// instead (`tiles`): rows per partition, items of 2 rows and tiles in us: 0.4
+// (Newtonian sphere) 283, 213; 5.9 (RK3 HLLC) 995, 942; 10 (wind) 1037, 1009,
+// (sphere) 984, 986; 20 (sphere) 1650, 1743.
+constexpr double F64_ROWS_OVER = 1.5, F64_ROWS_LEAST = 2.0, F64_ROWS_MOST = 16.0;
+constexpr double F64_WAVE_GRID = 12.0, F64_WAVE_ROWS = 8.0, F64_LARGE_GRID = 24.0;
 constexpr double F64_TILE_GRID = 8.0;
+
+// FP64 items by the grid (f64_items): the default tuning, tiles of 8 rows, of
+// the separate stage. Every other tile_rows, and strips, are as high as they say.
+bool f64_rows_by_grid(int32_t utr, int32_t uform) { return utr == 8 && uform != KNC_UPDATE_STRIP; }
 
 std::vector<int4> f64_items(const std::vector<std::pair<int64_t, int64_t>>& shapes, int slot0, int sms, bool& tiles) {
     double left = 0.0;   // rows of 32 columns left, per SM partition
     for (const auto& s : shapes) left += (double)(s.first * ((s.second + TILE_Q - 1) / TILE_Q)) / (4.0 * sms);
-    const double most = left < F64_ROWS_SMALL_GRID ? F64_ROWS_LEAST : F64_ROWS_MOST;
+    // the rows of an item: between `least` and `most`
+    const bool wave = left >= F64_WAVE_GRID && left < F64_LARGE_GRID;
+    const double least = wave ? F64_WAVE_ROWS : F64_ROWS_LEAST;
+    const double most = wave ? F64_WAVE_ROWS : left < F64_WAVE_GRID ? F64_ROWS_LEAST : F64_ROWS_MOST;
     std::vector<int4> items;
     tiles = left < F64_TILE_GRID;
     if (tiles) {
@@ -266,7 +278,7 @@ std::vector<int4> f64_items(const std::vector<std::pair<int64_t, int64_t>>& shap
     for (size_t k = 0; k < shapes.size(); ++k) {
         const int64_t nr = shapes[k].first, nq = shapes[k].second, cols = (nq + TILE_Q - 1) / TILE_Q;
         for (int64_t i0 = 0; i0 < nr;) {
-            const int64_t want = (int64_t)std::min(std::max(left / F64_ROWS_OVER, F64_ROWS_LEAST), most);
+            const int64_t want = (int64_t)std::min(std::max(left / F64_ROWS_OVER, least), most);
             const int64_t per = (nr - i0 + want - 1) / want, rows = (nr - i0 + per - 1) / per;
             for (int64_t j0 = 0; j0 < nq; j0 += TILE_Q)
                 items.push_back(make_int4(slot0 + (int)k, (int)i0, (int)j0, (int)rows));
@@ -513,7 +525,6 @@ struct knc_ctx {
     int32_t guess = KNC_GUESS_PLAIN;
     int32_t batched = 0;
     int32_t utr = 8;   // update tile rows (4, 8 or 16)
-    bool utr_set = false;   // chosen by the caller or the autotuner
     int32_t fused = 0;         // one cooperative launch per stage
     int32_t uform = KNC_UPDATE_TILE;   // update form of the separate stage
     int32_t rform = KNC_RECOVERY_INLINE;   // mixed recovery form of the separate stage
@@ -769,7 +780,7 @@ int rebuild_table(knc_ctx* c) {
     // the separate FP64 update takes items of 32 whole columns and at most 32
     // rows, in both update forms
     const bool rows64 = c->precision != KNC_PRECISION_MIXED && !c->fused;
-    const bool rows_auto = rows64 && !c->utr_set;
+    const bool rows_auto = rows64 && f64_rows_by_grid(c->utr, c->uform);
     const int cols = rows64 ? TILE_Q : STRIP_OUT;
     const bool guided = c->uform == KNC_UPDATE_STRIP && !rows64 && !c->fused;   // strips by mixed_strips
     if (!c->dirty && L(c).utr == c->utr && L(c).uform == c->uform && L(c).chunk_nt == fused_threads(c) &&
@@ -2881,7 +2892,6 @@ int knc_set_tuning(knc_ctx* c, const knc_tuning* t) {
     if (t->fused && !c->coop)
         return set_msg(c, KNC_ERR_UNSUPPORTED, "the device has no cooperative launch (fused stage)");
     c->utr = t->tile_rows;
-    c->utr_set = true;
     c->fused = t->fused ? 1 : 0;
     c->ctas_per_sm = t->ctas_per_sm;
     // the fused stage stages its tiles itself (no tensor-copy form)
@@ -2919,7 +2929,8 @@ int knc_autotune(knc_ctx* c, int32_t reps, knc_tuning* best_out, double* ms_out)
     if (c->mesh.p.num_polar_zones > 1)
         for (int sr : {4, 8, 10, 12, 16, 20, 24, 32, 64})
             for (int mb : {4, 5, 6})
-                if (mixed(c) || mb == 4) cands.push_back({sr, 0, mb, KNC_UPDATE_STRIP});
+                // (an FP64 item has 32 rows at most)
+                if (mixed(c) || (mb == 4 && sr <= 32)) cands.push_back({sr, 0, mb, KNC_UPDATE_STRIP});
     // The fused stages (one cooperative launch per stage) only for solvers
     // that launch their stages from the host one by one, the way candidates
     // are timed: inside a batched solver's captured folds, where the
@@ -2969,7 +2980,6 @@ int knc_autotune(knc_ctx* c, int32_t reps, knc_tuning* best_out, double* ms_out)
     for (size_t ci = 0; ci < cands.size(); ++ci) {
         const knc_tuning t = cands[ci];
         c->utr = t.tile_rows;
-        c->utr_set = true;
         c->fused = t.fused;
         c->ctas_per_sm = t.ctas_per_sm;
         c->uform = t.update_form;
@@ -3013,7 +3023,6 @@ int knc_autotune(knc_ctx* c, int32_t reps, knc_tuning* best_out, double* ms_out)
     c->stage_counter = 0;
     c->bar_epoch = 0;
     c->utr = best.tile_rows;
-    c->utr_set = true;
     c->fused = best.fused;
     c->ctas_per_sm = best.ctas_per_sm;
     c->uform = best.update_form;

@@ -108,7 +108,9 @@ class Solver:
     def set_tuning(self, tile_rows: int = 8, fused: bool = False, ctas_per_sm: int = 0, tma: bool = False,
                    strip: bool = False, deferred: bool = False):
         """Launch shape: update tiles of tile_rows rows (tma: staged by tensor
-        copies), warp strips of tile_rows rows (strip), or the fused stage."""
+        copies), warp strips of tile_rows rows (strip), or the fused stage. In
+        the separate FP64 stage the default (tiles of 8 rows) means rows that
+        follow the grid."""
         form = abi.KNC_UPDATE_STRIP if strip else abi.KNC_UPDATE_TILE_TMA if tma else abi.KNC_UPDATE_TILE
         t = abi.Tuning(tile_rows=int(tile_rows), fused=int(bool(fused)), ctas_per_sm=int(ctas_per_sm),
                        update_form=form, recovery_form=int(bool(deferred)))

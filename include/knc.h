@@ -266,7 +266,8 @@ int knc_set_batched(knc_ctx* ctx, int32_t graph);
  *                a tile runs on (tile_rows + 1) warps), or at most of a warp
  *                strip (4 to 64; lower towards the end of the grid). In the
  *                separate FP64 stage: rows of a warp's item of 32 columns (32
- *                at most; chosen by the grid while no tuning is set)
+ *                at most); tiles of 8, the default, are by the grid: items
+ *                whose rows follow the work left, or small tiles
  *   fused        0: a stage is four launches (ghost rows, recovery, remaps,
  *                update; the deferring recovery adds its dense pass); 1: one
  *                persistent cooperative launch whose phases are separated by
