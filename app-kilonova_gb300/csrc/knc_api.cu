@@ -22,6 +22,7 @@
 #include <cudaTypedefs.h>
 
 #include "knc_internal.h"
+#include "knc_runs.h"
 #include "knc_tma.cuh"
 
 using namespace knc;
@@ -322,52 +323,6 @@ std::vector<int4> mixed_strips(const std::vector<std::pair<int64_t, int64_t>>& s
     return strips;
 }
 
-// The row-walking recovery's runs {slot, i0, j0, rows}: the blocks' columns of
-// 32 zones, one after the other, cut into as many equal runs of whole rows as
-// the device holds warps of it (`off`: warp k's first run; a column's end cuts
-// too). A run's first rows wait for memory with nothing to compute, so a warp
-// has one or two, not one per tile, and all warps end together. Where a
-// block's columns fill CTAs, the warps of a CTA walk the same rows of
-// neighbouring columns. Against 8-row tiles strided over the same warps (4.5
-// tiles a warp on the 4096 x 1024 wind, 1.1 on the 2048 x 512 jet): folds of
-// 20 wind steps 9.93 -> 9.87 ms on the device (9.98 with every column on its
-// own), 10 jet steps 3.68 -> 3.53, 2 RK3 steps of uneven blocks 1.33 -> 1.28.
-void recovery_runs(const std::vector<std::pair<int64_t, int64_t>>& shapes, int sms, std::vector<int4>& runs,
-                   std::vector<int>& off) {
-    constexpr int WPC = TILE_THREADS / 32;
-    const int64_t resident = (int64_t)sms * C2P_ROWS_CTAS * WPC;
-    int64_t total = 0;
-    for (const auto& s : shapes) total += s.first * ((s.second + TILE_Q - 1) / TILE_Q);
-    const int64_t per = std::max<int64_t>(1, (total + resident - 1) / resident);
-    std::vector<std::vector<int4>> warps;
-    for (int width : {WPC, 1}) {
-        int64_t done = 0;   // rows given to each of `width` neighbouring warps
-        while (warps.size() % WPC) warps.emplace_back();   // whole CTAs
-        for (size_t k = 0; k < shapes.size(); ++k) {
-            const int64_t nr = shapes[k].first, nq = shapes[k].second, cols = (nq + TILE_Q - 1) / TILE_Q;
-            if ((cols % WPC == 0 ? WPC : 1) != width) continue;
-            for (int64_t j0 = 0; j0 < nq; j0 += width * TILE_Q)
-                for (int64_t i0 = 0; i0 < nr;) {
-                    if (done % per == 0) warps.resize(warps.size() + width);
-                    const int64_t rows = std::min(nr - i0, per - done % per);
-                    for (int w = 0; w < width; ++w)
-                        warps[warps.size() - width + w].push_back(
-                            make_int4((int)k, (int)i0, (int)(j0 + w * TILE_Q), (int)rows));
-                    i0 += rows;
-                    done += rows;
-                }
-        }
-    }
-    while (warps.size() % WPC) warps.emplace_back();
-    runs.clear();
-    off.clear();
-    for (const auto& w : warps) {
-        off.push_back((int)runs.size());
-        runs.insert(runs.end(), w.begin(), w.end());
-    }
-    off.push_back((int)runs.size());
-}
-
 // One block set's device view.
 struct Layout {
     DevBlock* d_table = nullptr;
@@ -392,6 +347,7 @@ struct Layout {
     int* d_run_off = nullptr;
     int run_off_cap = 0;
     int run_warps = 0;
+    bool runs_built = false;    // (only for the separate deferring mixed stage)
     int4* d_strips = nullptr;   // warp strips {slot, i0, j0, rows} of `utr` rows (strip form)
     int strips_cap = 0;
     int nstrips = 0;
@@ -783,8 +739,11 @@ int rebuild_table(knc_ctx* c) {
     const bool rows_auto = rows64 && f64_rows_by_grid(c->utr, c->uform);
     const int cols = rows64 ? TILE_Q : STRIP_OUT;
     const bool guided = c->uform == KNC_UPDATE_STRIP && !rows64 && !c->fused;   // strips by mixed_strips
+    // the row-walking recovery's runs, for the one stage form that launches it
+    const bool with_runs =
+        c->precision == KNC_PRECISION_MIXED && !c->fused && c->rform == KNC_RECOVERY_DEFERRED;
     if (!c->dirty && L(c).utr == c->utr && L(c).uform == c->uform && L(c).chunk_nt == fused_threads(c) &&
-        L(c).list_cols == cols && L(c).list_auto == (rows_auto || guided))
+        L(c).list_cols == cols && L(c).list_auto == (rows_auto || guided) && (!with_runs || L(c).runs_built))
         return KNC_OK;
     const int64_t item_rows = rows64 ? std::min<int64_t>(c->utr, 32) : c->utr;
     L(c).list_cols = cols;
@@ -954,26 +913,29 @@ int rebuild_table(knc_ctx* c) {
                            c->stream));
     L(c).nchunks = (int)chunks.size();
     L(c).chunk_nt = nt;
-    std::vector<int4> runs;
-    std::vector<int> run_off;
-    recovery_runs(shapes, c->sms, runs, run_off);
-    if ((int)runs.size() > L(c).runs_cap) {
-        cudaFree(L(c).d_runs);
-        L(c).d_runs = nullptr;
-        CK(dalloc(&L(c).d_runs, runs.size()));
-        L(c).runs_cap = (int)runs.size();
+    const RecoveryRuns runs =
+        with_runs ? recovery_runs(shapes, (int64_t)c->sms * C2P_ROWS_CTAS) : RecoveryRuns{};
+    if (with_runs) {
+        if ((int)runs.runs.size() > L(c).runs_cap) {
+            cudaFree(L(c).d_runs);
+            L(c).d_runs = nullptr;
+            CK(dalloc(&L(c).d_runs, runs.runs.size()));
+            L(c).runs_cap = (int)runs.runs.size();
+        }
+        if ((int)runs.off.size() > L(c).run_off_cap) {
+            cudaFree(L(c).d_run_off);
+            L(c).d_run_off = nullptr;
+            CK(dalloc(&L(c).d_run_off, runs.off.size()));
+            L(c).run_off_cap = (int)runs.off.size();
+        }
+        if (!runs.runs.empty())
+            CK(cudaMemcpyAsync(L(c).d_runs, runs.runs.data(), runs.runs.size() * sizeof(int4), cudaMemcpyHostToDevice,
+                               c->stream));
+        CK(cudaMemcpyAsync(L(c).d_run_off, runs.off.data(), runs.off.size() * sizeof(int), cudaMemcpyHostToDevice,
+                           c->stream));
     }
-    if ((int)run_off.size() > L(c).run_off_cap) {
-        cudaFree(L(c).d_run_off);
-        L(c).d_run_off = nullptr;
-        CK(dalloc(&L(c).d_run_off, run_off.size()));
-        L(c).run_off_cap = (int)run_off.size();
-    }
-    if (!runs.empty())
-        CK(cudaMemcpyAsync(L(c).d_runs, runs.data(), runs.size() * sizeof(int4), cudaMemcpyHostToDevice, c->stream));
-    CK(cudaMemcpyAsync(L(c).d_run_off, run_off.data(), run_off.size() * sizeof(int), cudaMemcpyHostToDevice,
-                       c->stream));
-    L(c).run_warps = (int)run_off.size() - 1;
+    L(c).run_warps = with_runs ? (int)runs.off.size() - 1 : 0;
+    L(c).runs_built = with_runs;
     if ((int)strips.size() > L(c).strips_cap) {
         cudaFree(L(c).d_strips);
         L(c).d_strips = nullptr;
