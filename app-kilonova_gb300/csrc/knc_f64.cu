@@ -94,7 +94,7 @@ struct F64C2p {
 template <bool MLP>
 __global__ void __launch_bounds__(TILE_THREADS, MLP ? 1 : 4) c2p_f64_kernel(StageArgs a) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
-    if (cta_any(stopped_before(a))) return;
+    const bool run = !stopped_before(a);
     MlpWeights& W = *reinterpret_cast<MlpWeights*>(smem_raw);
     __nv_bfloat16* act = reinterpret_cast<__nv_bfloat16*>(smem_raw + sizeof(MlpWeights)) +
                          (threadIdx.x >> 5) * MLP_ACT_ELEMS;
@@ -103,7 +103,7 @@ __global__ void __launch_bounds__(TILE_THREADS, MLP ? 1 : 4) c2p_f64_kernel(Stag
         __syncthreads();
     }
     C2pStats st;
-    for (int tile = blockIdx.x; tile < a.ntiles; tile += gridDim.x) {
+    for (int tile = blockIdx.x; run && tile < a.ntiles; tile += gridDim.x) {
         const int4 t = a.tiles[tile];
         const DevBlock& B = a.blocks[t.x];
         const int i = t.y + threadIdx.x / TILE_Q;

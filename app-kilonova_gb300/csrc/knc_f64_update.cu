@@ -319,7 +319,6 @@ template <bool SRHD, bool HLLC>
 __global__ void __launch_bounds__(ROWS64_WARPS * 32, 3)
     update_tile64_kernel(const __grid_constant__ StageArgs a, const int4* __restrict__ items) {
     __shared__ Tile64 T;
-    if (cta_any(stopped(a))) return;
     const PhysT<double> ph = make_phys<double>(a);
     const int4 it = items[blockIdx.x];
     const DevBlock& B = a.blocks[it.x];
@@ -340,7 +339,8 @@ __global__ void __launch_bounds__(ROWS64_WARPS * 32, 3)
         }
         if (threadIdx.x == 0) T.claim = ROWS64_WARPS;
     }
-    __syncthreads();
+    // after a failure the CTA leaves as one (the barrier is needed anyway)
+    if (__syncthreads_or(stopped(a))) return;
     const unsigned polar = one_d ? 0u : (unsigned)rows, passes = polar + (unsigned)rows + 1u;
     const int j = j0 + lane;
     // A warp's first pass is rotated with the CTA: a warp stays on its SM

@@ -351,8 +351,7 @@ struct MixedC2p {
 template <bool MLP>
 __global__ void __launch_bounds__(TILE_THREADS, 3) c2p_mixed_kernel(StageArgs a) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
-    const bool stop = stopped_before(a);
-    if (MLP ? cta_any(stop) : stop) return;   // (the warps meet where they load the weights)
+    const bool run = !stopped_before(a);
     MlpWeights& W = *reinterpret_cast<MlpWeights*>(smem_raw);
     __nv_bfloat16* act = reinterpret_cast<__nv_bfloat16*>(smem_raw + sizeof(MlpWeights)) +
                          (threadIdx.x >> 5) * MLP_ACT_ELEMS;
@@ -361,7 +360,7 @@ __global__ void __launch_bounds__(TILE_THREADS, 3) c2p_mixed_kernel(StageArgs a)
         __syncthreads();
     }
     C2pStats st;
-    for (int tile = blockIdx.x; tile < a.ntiles; tile += gridDim.x) {
+    for (int tile = blockIdx.x; run && tile < a.ntiles; tile += gridDim.x) {
         const int4 t = a.tiles[tile];
         const DevBlock& B = a.blocks[t.x];
         const int i = t.y + threadIdx.x / TILE_Q;

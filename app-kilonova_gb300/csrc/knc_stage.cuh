@@ -89,12 +89,12 @@ __device__ __forceinline__ R stage_plm(R theta, R a, R b, R c) {
     else return plm_gradient(theta, a, b, c);
 }
 
-// Whether a failure stops a launch that works on `stage` (recovery: one of an
+// Whether a failure stops a launch that works on a.stage (recovery: one of an
 // earlier stage; update: any). The chunks of a host-state step run on several
-// streams, so another chunk's failure can appear while a CTA starts: a kernel
-// with barriers or sums over its CTA asks once per CTA (every thread calls
-// it), or some of its warps would leave and the others read shared words that
-// nobody wrote.
+// streams, so another chunk's failure can appear while a CTA starts and its
+// warps can answer differently: a kernel with barriers, shared words or sums
+// over its CTA keeps all its warps (the recoveries skip their tiles, the FP64
+// tile update leaves as one).
 __device__ __forceinline__ bool stopped_before(const StageArgs& a) {
     const unsigned long long ek = *(volatile const unsigned long long*)&a.status->err_key;
     return ek != NO_ERROR && (uint32_t)(ek >> 48) < (uint32_t)a.stage;
@@ -102,7 +102,6 @@ __device__ __forceinline__ bool stopped_before(const StageArgs& a) {
 __device__ __forceinline__ bool stopped(const StageArgs& a) {
     return *(volatile const unsigned long long*)&a.status->err_key != NO_ERROR;
 }
-__device__ __forceinline__ bool cta_any(bool x) { return __syncthreads_or(x) != 0; }
 
 // The stage's time step: the host's dt, or (adaptive dt found on the device)
 // the reduced dl / a_max times the CFL number, formed like the host would.
