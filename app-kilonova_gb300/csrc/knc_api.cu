@@ -330,7 +330,7 @@ struct Layout {
     int4* d_tiles = nullptr;
     int tiles_cap = 0;
     int ntiles = 0;
-    int4* d_utiles = nullptr;   // update tiles of `utr` rows
+    int4* d_utiles = nullptr;   // update tiles of `utr` rows, or the FP64 update's items
     int utiles_cap = 0;
     int nutiles = 0;
     int utr = 0;
@@ -480,7 +480,7 @@ struct knc_ctx {
     int32_t precision = KNC_PRECISION_FP64;
     int32_t guess = KNC_GUESS_PLAIN;
     int32_t batched = 0;
-    int32_t utr = 8;   // update tile rows (4, 8 or 16)
+    int32_t utr = 8;   // update tile rows (4, 8 or 16) or strip rows (4 to 64)
     int32_t fused = 0;         // one cooperative launch per stage
     int32_t uform = KNC_UPDATE_TILE;   // update form of the separate stage
     int32_t rform = KNC_RECOVERY_INLINE;   // mixed recovery form of the separate stage
@@ -1128,8 +1128,8 @@ StageArgs base_args(knc_ctx* c) {
     a.blocks = L(c).d_table;
     a.tiles = L(c).d_tiles;
     a.ntiles = L(c).ntiles;
-    a.runs = L(c).d_runs;
-    a.run_off = L(c).d_run_off;
+    a.runs = L(c).runs_built ? L(c).d_runs : nullptr;
+    a.run_off = L(c).runs_built ? L(c).d_run_off : nullptr;
     a.run_warps = L(c).run_warps;
     a.utiles = L(c).d_utiles;
     a.nutiles = L(c).nutiles;
@@ -2639,8 +2639,11 @@ int stream_step(knc_ctx* c, double dt, const double* hc_in, const double* hs_in,
             y.tiles = tiles;
             y.ntiles = ntiles;
             y.runs = nullptr;   // (they cover the whole layout)
-            // the update as warp strips of STREAM_STRIP_ROWS rows, whatever
-            // the tuned form (every form gives the same state)
+            y.run_off = nullptr;
+            y.run_warps = 0;
+            // the update as warp strips of STREAM_STRIP_ROWS rows (mixed), or
+            // as f64_items' items or tiles of the chunk (FP64), whatever the
+            // tuned form (every form gives the same state)
             y.strips = lay.d_sc_strips + lay.sc_strip_off[k * S + s];
             y.nstrips = lay.sc_strip_off[k * S + s + 1] - lay.sc_strip_off[k * S + s];
             y.f64_tiles = lay.list_cols == TILE_Q ? lay.sc_tiles64[k] : 0;
@@ -2742,7 +2745,7 @@ int knc_advance_host(knc_ctx* c, const double* cons_in, const double* scalar_in,
     const bool adaptive = !(c->hp.system == KNC_SYSTEM_RELATIVISTIC && !c->hp.adaptive_time_step);
     const bool pinned = device_view(cons_in) && device_view(scalar_in) && device_view(cons_out) &&
                         device_view(scalar_out);
-    // (the chunks update as warp strips, which need a polar grid)
+    // (mixed chunks update as warp strips, which need a polar grid)
     const bool streamed = pinned && fold > 0 && !adaptive && !c->fused && L(c).nremap == 0 &&
                           c->model.kind != KNC_MODEL_HOST && c->mesh.p.num_polar_zones > 1 &&
                           chunks_fit(L(c), c->hp.runge_kutta_order, most_chunks(c));

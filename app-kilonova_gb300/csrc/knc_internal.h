@@ -116,7 +116,8 @@ struct StageArgs {
     const DevBlock* blocks;
     const int4* tiles;      // {slot, i0, j0, 0}, TILE_R x TILE_Q (recovery, init)
     int32_t ntiles;
-    const int4* utiles;     // {slot, i0, j0, rows}, utr x TILE_Q (update)
+    const int4* utiles;     // {slot, i0, j0, rows} (update): utr x TILE_Q tiles; separate FP64 stage: items
+                            // of TILE_Q columns, or tiles of TILE64_COLS (f64_tiles), of the rows they say
     int32_t nutiles;
     int32_t utr;            // update tile rows: 4, 8 or 16
     int32_t tma;            // mixed update: stage tiles with tensor copies (tmaps valid)
@@ -173,7 +174,7 @@ struct StageArgs {
     unsigned* high_count;       // this stage's count (status word, by stage parity)
     unsigned* high_count_next;  // the next stage's, cleared by the dense pass
     unsigned high_cap;          // entries a.high holds
-    // row-walking recovery: the runs {slot, i0, j0, rows} of 32 columns that warp
+    // row-walking recovery (knc_runs.h; null elsewhere): the runs {slot, i0, j0, rows} of 32 columns that warp
     // k walks are runs[run_off[k]] .. runs[run_off[k + 1] - 1], for run_warps
     // warps (a multiple of a CTA's)
     const int4* runs;

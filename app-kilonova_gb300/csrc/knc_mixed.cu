@@ -3,7 +3,7 @@
 // Same method as the FP64 stage (src/scheme.rs:16-173), with the precision
 // moved per operation:
 //   FP32  reconstruction, Riemann fluxes, geometric sources, geometry factors
-//         (update_kernel<float, true>), primitive storage;
+//         (update_kernel, update_strip_kernel), primitive storage;
 //   FP64  the conserved state and its RK accumulation, time and excision
 //         radius (host), and the cons -> prim recovery of zones whose Lorentz
 //         factor exceeds `w_split` — converged to the reference's residual
@@ -556,7 +556,7 @@ cudaError_t launch_c2p_mixed(const StageArgs& a, cudaStream_t s) {
     if (a.ntiles <= 0) return cudaSuccess;
     if (a.high) {
         // every zone in FP32; the ones that need the FP64 recovery, densely after
-        // one resident grid, a warp per entry of a.run_off
+        // (a warp per entry of a.run_off, all CTAs resident)
         auto k = a.compute_dt ? c2p_rows_kernel<1> : c2p_rows_kernel<0>;
         cudaError_t e = launch_chained(k, a.run_warps / (TILE_THREADS / 32), TILE_THREADS, 0, s, a);
         if (e != cudaSuccess) return e;
@@ -676,8 +676,8 @@ static void update_mixed(const StageArgs& a, cudaStream_t s) {
         return;
     }
     const size_t smem = StageSmem<float, TR>::bytes;
-    const int grid = std::min(a.nutiles, resident_grid(update_kernel<float, true, TR>, update_threads<TR>(), smem));
-    update_kernel<float, true, TR><<<grid, update_threads<TR>(), smem, s>>>(a);
+    const int grid = std::min(a.nutiles, resident_grid(update_kernel<TR>, update_threads<TR>(), smem));
+    update_kernel<TR><<<grid, update_threads<TR>(), smem, s>>>(a);
 }
 
 template <int MB>
@@ -685,7 +685,7 @@ static void update_strips(const StageArgs& a, cudaStream_t s) {
     // (with a list at least one CTA per SM: its zones are claimed by every warp)
     const int want = std::max((a.nstrips + STRIP_WARPS - 1) / STRIP_WARPS, a.hp_list ? num_sms() : 1);
     // a CTA of warps per STRIP_WARPS strips, taken by the SMs as they come free
-    launch_chained(update_strip_kernel<float, true, MB>, want, STRIP_WARPS * 32, 0, s, a);
+    launch_chained(update_strip_kernel<MB>, want, STRIP_WARPS * 32, 0, s, a);
 }
 
 cudaError_t launch_update_mixed(const StageArgs& a, cudaStream_t s) {
@@ -709,7 +709,7 @@ cudaError_t launch_update_mixed(const StageArgs& a, cudaStream_t s) {
 
 template <int TR>
 static cudaError_t configure_update_mixed() {
-    cudaError_t e = cudaFuncSetAttribute(update_kernel<float, true, TR>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+    cudaError_t e = cudaFuncSetAttribute(update_kernel<TR>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                          (int)StageSmem<float, TR>::bytes);
     if (e != cudaSuccess) return e;
     return cudaFuncSetAttribute(update_tma_kernel<TR>, cudaFuncAttributeMaxDynamicSharedMemorySize,

@@ -386,21 +386,20 @@ __device__ __forceinline__ void update_tile(const StageArgs& a, const int4 t, un
     }
 }
 
-// Update tiles (a.utiles) in a grid-stride loop: the launch is sized to the
+// The mixed stage's update tiles (a.utiles) in a grid-stride loop: the launch is sized to the
 // resident CTAs, so no CTA pays start-up per tile.
-template <class R, bool MIXED, int TR>
-__global__ void __launch_bounds__(update_threads<TR>(), MIXED ? (TR == 4 ? 6 : TR == 8 ? 3 : 2) : 1)
-    update_kernel(StageArgs a) {
+template <int TR>
+__global__ void __launch_bounds__(update_threads<TR>(), TR == 4 ? 6 : TR == 8 ? 3 : 2) update_kernel(StageArgs a) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     // A failed c2p in this or an earlier stage stops the step: keep the
     // input state untouched so the failure can be reported from it.
     if (*(volatile unsigned long long*)&a.status->err_key != NO_ERROR) return;
-    if constexpr (MIXED) clear_next_hp(a);
+    clear_next_hp(a);
     for (int tile = blockIdx.x; tile < a.nutiles; tile += gridDim.x) {
-        update_tile<R, MIXED, TR>(a, a.utiles[tile], smem_raw);
+        update_tile<float, true, TR>(a, a.utiles[tile], smem_raw);
         __syncthreads();
     }
-    if constexpr (MIXED) drain_hp(a);
+    drain_hp(a);
 }
 
 // ---- warp strips ---------------------------------------------------------------
@@ -965,19 +964,19 @@ __device__ __forceinline__ void stage_strips(const StageArgs& a, int first, int 
     for (int k = first; k < a.nstrips; k += step) update_strip<R, MIXED>(a, a.strips[k], ph);
 }
 
-// Strips (a.strips), one to a warp; MB = resident CTAs per SM the register
+// The mixed stage's strips (a.strips), one to a warp; MB = resident CTAs per SM the register
 // allocation is sized for (a tuning choice: more warps against fewer
 // registers). A resident grid striding over the strips was measured too, at
 // strips of even height: 12.05 against 12.16 ms (4096 x 1024 wind fold); with
 // the heights of mixed_strips 11.92 against 11.73.
-template <class R, bool MIXED, int MB>
+template <int MB>
 __global__ void __launch_bounds__(STRIP_WARPS * 32, MB) update_strip_kernel(const __grid_constant__ StageArgs a) {
     // launched chained to the recovery (programmatic dependent launch): wait
     // for it to complete, let the next stage's recovery be scheduled
     asm volatile("griddepcontrol.wait;" ::: "memory");
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     if (*(volatile unsigned long long*)&a.status->err_key != NO_ERROR) return;
-    stage_strips<R, MIXED>(a, blockIdx.x * STRIP_WARPS + (threadIdx.x >> 5), gridDim.x * STRIP_WARPS);
+    stage_strips<float, true>(a, blockIdx.x * STRIP_WARPS + (threadIdx.x >> 5), gridDim.x * STRIP_WARPS);
 }
 
 // Block-wide reduction helpers (warp shuffles, then one atomic per warp).
